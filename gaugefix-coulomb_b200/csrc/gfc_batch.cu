@@ -99,6 +99,7 @@ struct BState {
 // ------------------------------------------------------------------ compaction --
 // One block.  Builds the three work lists from the state table.
 __global__ void __launch_bounds__(1024) k_compact(BState b) {
+    grid_wait();
     __shared__ int sc[4][1024];
     __shared__ int sact[1024];
     const int tid = threadIdx.x;
@@ -183,6 +184,7 @@ __device__ __forceinline__ void slot_fields(const BSlot &sl, typename S::V *&u, 
 // shared memory of 6 x NS x BCHUNK x 16 bytes), as in the single-lattice kernel
 template <class S, int MINB, bool STG>
 __global__ void __launch_bounds__(BCHUNK, MINB) k_bsweep(BState b) {
+    grid_wait();
     extern __shared__ __align__(16) unsigned char bstage[];
     using T = typename S::T;
     constexpr bool F64 = sizeof(T) == 8;
@@ -338,6 +340,7 @@ struct Handout {
 // of the shared array in both precisions' layouts.
 template <int MINB>
 __global__ void __launch_bounds__(32, MINB) k_bsweep_wf(BState b) {
+    grid_wait();
     extern __shared__ __align__(16) unsigned char bstage[];
     const int n32 = b.counts[0];
     const Handout h(n32 + b.counts[1]);
@@ -364,6 +367,7 @@ __global__ void __launch_bounds__(32, MINB) k_bsweep_wf(BState b) {
 
 template <class S, int MINB>
 __global__ void __launch_bounds__(32, MINB) k_bsweep_w(BState b) {
+    grid_wait();
     extern __shared__ __align__(16) unsigned char bstage[];
     constexpr bool F64 = sizeof(typename S::T) == 8;
     const Handout h(b.counts[F64 ? 1 : 0]);
@@ -406,6 +410,7 @@ __device__ __forceinline__ bool odd_parity_site_t(const Lat &l, int p, uint32_t 
 // consecutive levels in the sequential sweep's order (see SS_LEX).
 template <int MINB>
 __global__ void __launch_bounds__(32, MINB) k_bsweep_lex(BState b, int level) {
+    grid_wait();
     extern __shared__ __align__(16) unsigned char bstage[];
     const int n = b.counts[10] * BPIECES;
     int *cursor = b.counts + 11 + level;
@@ -449,6 +454,7 @@ __global__ void __launch_bounds__(32, MINB) k_bsweep_lex(BState b, int level) {
 // e2 of the odd-ns timeslices measured on this half-sweep (mflag MF_NOW), over all
 // their sites, on the state the four level launches left: one partial per piece.
 __global__ void __launch_bounds__(32) k_bmeasure_lex(BState b) {
+    grid_wait();
     const int n = b.counts[10];
     int *cursor = b.counts + 15;
     const int lane = threadIdx.x;
@@ -488,6 +494,7 @@ __global__ void __launch_bounds__(32) k_bmeasure_lex(BState b) {
 // previous half-sweep and retires it: FP32 -> pending switch at the switch
 // threshold, FP64 -> done at the tolerance, NaN -> done with the status bit.
 __global__ void k_bslice(BState b) {
+    grid_wait();
     const int lane = threadIdx.x & 31;
     // both sweep kernels of this half-sweep have finished: count it and reset their
     // item cursors for the next one
@@ -664,6 +671,7 @@ __device__ __forceinline__ void breunit_part(const BState &b, unsigned period, i
 }
 
 __global__ void __launch_bounds__(BCHUNK) k_breunit(BState b) {
+    grid_wait();
     __shared__ int due[BCHUNK];
     __shared__ int ndue;
     breunit_part<S32>(b, b.reunit32, due, ndue);
@@ -680,6 +688,7 @@ __global__ void __launch_bounds__(BCHUNK) k_breunit(BState b) {
 // BCHUNK FP32 items at once and rebuilds the chunks of due timeslices only.
 template <int PASS>
 __global__ void __launch_bounds__(BCHUNK) k_brefresh(BState b) {
+    grid_wait();
     __shared__ int due[BCHUNK];
     __shared__ int ndue;
     if (!b.refresh32 || !b.counts[16]) return;   // uniform
@@ -742,6 +751,7 @@ __global__ void __launch_bounds__(BCHUNK) k_brefresh(BState b) {
 // --------------------------------------------------- FP32 -> FP64 switch --
 // pass 1: G in FP64 (row 2 rebuilt from the FP32 rows, projected) into g and g64r
 __global__ void __launch_bounds__(BCHUNK) k_switch_g(BState b) {
+    grid_wait();
     const int n = b.counts[2];
     for (int it = blockIdx.x; it < n; it += gridDim.x) {
         const int2 item = b.pend[it];
@@ -771,6 +781,7 @@ __global__ void __launch_bounds__(BCHUNK) k_switch_g(BState b) {
 
 // pass 2: links U_d(x) = G(x) U0_d(x) G(x+d)^dagger from the FP64 originals into u64r
 __global__ void __launch_bounds__(BCHUNK) k_switch_u(BState b) {
+    grid_wait();
     const int n = b.counts[2];
     for (int it = blockIdx.x; it < n; it += gridDim.x) {
         const int2 item = b.pend[it];
@@ -800,6 +811,7 @@ __global__ void __launch_bounds__(BCHUNK) k_switch_u(BState b) {
 
 // pass 3: pending timeslices become FP64; the previous e2 entry is invalidated
 __global__ void k_switch_done(BState b) {
+    grid_wait();
     const int gid = blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= b.nslices || b.state[gid] != SS_PEND) return;
     b.state[gid] = SS_FP64;
@@ -811,6 +823,7 @@ __global__ void k_switch_done(BState b) {
 
 // activate the timeslices of one slot in `state`
 __global__ void k_activate(BState b, int gid0, int nt, int state) {
+    grid_wait();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nt) return;
     const int gid = gid0 + t;
@@ -825,6 +838,7 @@ __global__ void k_activate(BState b, int gid0, int nt, int state) {
 }
 
 __global__ void k_set_state(int *state, int gid0, int nt, int value) {
+    grid_wait();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < nt) state[gid0 + t] = value;
 }
@@ -1190,7 +1204,7 @@ extern "C" int gfc_batch_activate(gfc_batch *b, int slot, int precision) {
     bs.ring = b->ring;
     bs.mflag = b->mflag;
     bs.mk = b->mk;
-    k_activate<<<(l.nt + 127) / 128, 128, 0, b->s>>>(bs, slot * b->max_nt, l.nt, st);
+    launch_early(k_activate, (l.nt + 127) / 128, 128, 0, b->s, bs, slot * b->max_nt, l.nt, st);
     b->launches += 5;
     b->activated[slot] = 1;
     GFC_CHECK(cudaGetLastError());
@@ -1240,7 +1254,7 @@ static void launch_bsweep_k(int grid, cudaStream_t st, const BState &bs) {
         static std::atomic<unsigned long long> done{0};
         smem_attr_once(done, kern, bytes);
     }
-    kern<<<grid, BCHUNK, bytes, st>>>(bs);
+    launch_early(kern, grid, BCHUNK, bytes, st, bs);
 }
 
 static void launch_bsweep_lex(int grid, cudaStream_t st, const BState &bs, int level) {
@@ -1248,7 +1262,7 @@ static void launch_bsweep_lex(int grid, cudaStream_t st, const BState &bs, int l
     auto kern = k_bsweep_lex<11>;
     static std::atomic<unsigned long long> done{0};
     smem_attr_once(done, kern, bytes);
-    kern<<<grid, 32, bytes, st>>>(bs, level);
+    launch_early(kern, grid, 32, bytes, st, bs, level);
 }
 
 template <int MINB>
@@ -1257,7 +1271,7 @@ static void launch_bsweep_wf_k(int grid, cudaStream_t st, const BState &bs) {
     auto kern = k_bsweep_wf<MINB>;
     static std::atomic<unsigned long long> done{0};
     smem_attr_once(done, kern, bytes);
-    kern<<<grid, 32, bytes, st>>>(bs);
+    launch_early(kern, grid, 32, bytes, st, bs);
 }
 
 // both precisions in one launch of one-warp CTAs, minb (8, 11 or 12) per SM
@@ -1275,7 +1289,7 @@ static void launch_bsweep_w(int grid, cudaStream_t st, const BState &bs) {
     auto kern = k_bsweep_w<S, MINB>;
     static std::atomic<unsigned long long> done{0};
     smem_attr_once(done, kern, bytes);
-    kern<<<grid, 32, bytes, st>>>(bs);
+    launch_early(kern, grid, 32, bytes, st, bs);
 }
 
 // minb: minimum resident CTAs per SM: 1..4 CTAs of BCHUNK threads (stage: FP64 links
@@ -1309,10 +1323,10 @@ static void launch_bsweep(int minb, bool stage, int grid, cudaStream_t st, const
 // enqueue one round on the stream (used for capture)
 static void enqueue_round(gfc_batch *b, const BState &bs) {
     cudaStream_t st = b->s;
-    k_compact<<<1, 1024, 0, st>>>(bs);
-    k_switch_g<<<b->grid, BCHUNK, 0, st>>>(bs);
-    k_switch_u<<<b->grid, BCHUNK, 0, st>>>(bs);
-    k_switch_done<<<(b->nslices + 255) / 256, 256, 0, st>>>(bs);
+    launch_early(k_compact, 1, 1024, 0, st, bs);
+    launch_early(k_switch_g, b->grid, BCHUNK, 0, st, bs);
+    launch_early(k_switch_u, b->grid, BCHUNK, 0, st, bs);
+    launch_early(k_switch_done, (b->nslices + 255) / 256, 256, 0, st, bs);
     for (int k = 0; k < b->round_k; k++) {
         // one resident wave of persistent CTAs: a CTA that had to wait for a slot
         // would start its share of the items late and stretch the tail
@@ -1327,13 +1341,13 @@ static void enqueue_round(gfc_batch *b, const BState &bs) {
         if (bs.lex) {
             // odd-ns timeslices: the four boundary levels in order, then their e2
             for (int level = 0; level < 4; level++) launch_bsweep_lex(b->nsm * 11, st, bs, level);
-            k_bmeasure_lex<<<b->nsm * 16, 32, 0, st>>>(bs);
+            launch_early(k_bmeasure_lex, b->nsm * 16, 32, 0, st, bs);
         }
-        k_bslice<<<(b->nslices + 7) / 8, 256, 0, st>>>(bs);
-        k_breunit<<<b->grid, BCHUNK, 0, st>>>(bs);
+        launch_early(k_bslice, (b->nslices + 7) / 8, 256, 0, st, bs);
+        launch_early(k_breunit, b->grid, BCHUNK, 0, st, bs);
         if (bs.refresh32) {
-            k_brefresh<0><<<b->grid, BCHUNK, 0, st>>>(bs);
-            k_brefresh<1><<<b->grid, BCHUNK, 0, st>>>(bs);
+            launch_early(k_brefresh<0>, b->grid, BCHUNK, 0, st, bs);
+            launch_early(k_brefresh<1>, b->grid, BCHUNK, 0, st, bs);
         }
     }
 }
@@ -1408,7 +1422,7 @@ extern "C" int gfc_batch_finalize(gfc_batch *b, int slot, gfc_report *r) {
     GFC_CHECK(cudaSetDevice(b->dev));
     const BSlot &sl = b->hs[slot];
     const Lat &l = sl.l;
-    k_set_state<<<(l.nt + 127) / 128, 128, 0, b->s>>>(b->state, slot * b->max_nt, l.nt, SS_DONE);
+    launch_early(k_set_state, (l.nt + 127) / 128, 128, 0, b->s, b->state, slot * b->max_nt, l.nt, SS_DONE);
     launch_unpack2(sl.u64r, sl.u, l.vh, 3 * l.npar, b->s);
     launch_unpack2(sl.g64r, sl.g, l.vh, l.npar, b->s);
     launch_reunitarize(sl.u, l.vh, 3 * l.npar, b->status, b->s);
@@ -1694,7 +1708,7 @@ extern "C" int gfc_batch_autotune(gfc_batch *b, int ns, int nt, double *times) {
     } while (0);
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
-    k_set_state<<<(nt + 127) / 128, 128, 0, b->s>>>(b->state, slot * b->max_nt, nt, SS_EMPTY);
+    launch_early(k_set_state, (nt + 127) / 128, 128, 0, b->s, b->state, slot * b->max_nt, nt, SS_EMPTY);
     b->activated[slot] = 0;
     int rc2 = gfc_batch_remove(b, slot);
     if (!rc) rc = rc2;

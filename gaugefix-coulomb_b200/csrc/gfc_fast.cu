@@ -184,6 +184,7 @@ template <class S, int BLOCK, int MINB>
 __global__ void __launch_bounds__(BLOCK, MINB) k_sweep_fast(typename S::V *__restrict__ u,
                                                             typename S::V *__restrict__ g, SweepArgs a) {
     using T = typename S::T;
+    grid_wait();
     if (a.stop && *(volatile unsigned *)a.stop) return;
     const Lat &l = a.l;
     const uint32_t vsh = l.vs >> 1;
@@ -201,6 +202,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_sweep_staged(typename S::V *__r
                                                               typename S::V *__restrict__ g, SweepArgs a) {
     extern __shared__ __align__(16) unsigned char staged_smem[];
     using T = typename S::T;
+    grid_wait();
     if (a.stop && *(volatile unsigned *)a.stop) return;
     const Lat &l = a.l;
     const uint32_t vsh = l.vs >> 1;
@@ -225,6 +227,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_sweep_staged(typename S::V *__r
 template <class S>
 __global__ void k_reunit_fast(typename S::V *__restrict__ base, uint32_t stride, uint32_t nblk, uint32_t begin,
                               uint32_t count, const unsigned *stop, unsigned *status) {
+    grid_wait();
     if (stop && *(volatile const unsigned *)stop) return;
     uint32_t j = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
     if (j >= count || k >= nblk) return;
@@ -238,6 +241,7 @@ __global__ void k_reunit_fast(typename S::V *__restrict__ base, uint32_t stride,
 
 // FP64 full SoA -> FP32 two-row SoA (nblk blocks of [9][stride] -> [3][stride])
 __global__ void k_to_f32(const double2 *__restrict__ src, float4 *__restrict__ dst, uint32_t stride, uint32_t nblk) {
+    grid_wait();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
     if (i >= stride || k >= nblk) return;
     const double2 *p = src + (size_t)k * 9 * stride + i;
@@ -252,6 +256,7 @@ __global__ void k_to_f32(const double2 *__restrict__ src, float4 *__restrict__ d
 
 // FP32 two-row SoA -> FP64 full SoA, row 2 rebuilt and the result projected in FP64
 __global__ void k_to_f64(const float4 *__restrict__ src, double2 *__restrict__ dst, uint32_t stride, uint32_t nblk) {
+    grid_wait();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
     if (i >= stride || k >= nblk) return;
     const float4 *p = src + (size_t)k * 3 * stride + i;
@@ -271,6 +276,7 @@ __global__ void k_to_f64(const float4 *__restrict__ src, double2 *__restrict__ d
 
 // FP64 full SoA ([9][stride] per block) -> FP64 two-row SoA ([6][stride])
 __global__ void k_pack2(const double2 *__restrict__ src, double2 *__restrict__ dst, uint32_t stride, uint32_t nblk) {
+    grid_wait();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
     if (i >= stride || k >= nblk) return;
     const double2 *p = src + (size_t)k * 9 * stride + i;
@@ -281,6 +287,7 @@ __global__ void k_pack2(const double2 *__restrict__ src, double2 *__restrict__ d
 
 // FP64 two-row -> full, row 2 = conj(row0 x row1)
 __global__ void k_unpack2(const double2 *__restrict__ src, double2 *__restrict__ dst, uint32_t stride, uint32_t nblk) {
+    grid_wait();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
     if (i >= stride || k >= nblk) return;
     Mt<double> m;
@@ -320,6 +327,7 @@ __global__ void k_round_check(const double *__restrict__ ring, int ring_n, int n
 }
 
 __global__ void k_identity32(float4 *__restrict__ g, uint32_t stride, uint32_t nblk) {
+    grid_wait();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
     if (i >= stride || k >= nblk) return;
     float4 *q = g + (size_t)k * 3 * stride + i;
@@ -336,6 +344,7 @@ __global__ void k_identity32(float4 *__restrict__ g, uint32_t stride, uint32_t n
 // composed with the transformation of the FP32 phase; with reset32 the FP32 G
 // restarts from the identity (as k_identity32 sets it).
 __global__ void k_compose_gt(float4 *__restrict__ g32, double2 *__restrict__ g, uint32_t stride, int reset32) {
+    grid_wait();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
     if (i >= stride) return;
     float4 *q = g32 + (size_t)k * 3 * stride + i;
@@ -377,6 +386,7 @@ __device__ __forceinline__ void store_rows01(double2 *__restrict__ p, size_t st,
 template <class S>
 __global__ void __launch_bounds__(128) k_regauge(const double2 *__restrict__ u0, const double2 *__restrict__ g,
                                                  typename S::V *__restrict__ out, Lat l) {
+    grid_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const int par = blockIdx.y;
     if (i >= l.vh) return;
@@ -434,7 +444,7 @@ static void launch_shape(dim3 grid, cudaStream_t st, typename S::V *u, typename 
     constexpr int B = kShapes[K].block;
     static_assert(B >= MIN_BLOCK, "block partial buffers are sized for MIN_BLOCK");
     grid.x = ((a.l.vs >> 1) + B - 1) / B;
-    k_sweep_fast<S, B, kShapes[K].minb><<<grid, B, 0, st>>>(u, g, a);
+    launch_early(k_sweep_fast<S, B, kShapes[K].minb>, grid, B, 0, st, u, g, a);
 }
 
 template <class S>
@@ -457,11 +467,11 @@ static void launch_staged(dim3 grid, cudaStream_t st, typename S::V *u, typename
             auto kp = k_sweep_staged<S, sh.block, sh.minb, (bool)sh.sg, sh.nst, true>;
             static std::atomic<unsigned long long> done_p{0};
             smem_attr_once(done_p, kp, bytes);
-            kp<<<grid, sh.block, bytes, st>>>(u, g, a);
+            launch_early(kp, grid, sh.block, bytes, st, u, g, a);
             return;
         }
     }
-    kern<<<grid, sh.block, bytes, st>>>(u, g, a);
+    launch_early(kern, grid, sh.block, bytes, st, u, g, a);
 }
 
 // Whether a half-sweep launched with SweepArgs::proj projects the links it writes
@@ -552,30 +562,30 @@ static int ensure_2row(gfc_ctx *c) {
 static void pack_2row(gfc_ctx *c) {
     const Lat &l = c->lat;
     dim3 gu((l.vh + 255) / 256, 3 * l.npar), gg((l.vh + 255) / 256, l.npar);
-    k_pack2<<<gu, 256, 0, c->s>>>(c->u, c->u64r, l.vh, 3 * l.npar);
-    k_pack2<<<gg, 256, 0, c->s>>>(c->g, c->g64r, l.vh, l.npar);
+    launch_early(k_pack2, gu, 256, 0, c->s, c->u, c->u64r, l.vh, 3 * l.npar);
+    launch_early(k_pack2, gg, 256, 0, c->s, c->g, c->g64r, l.vh, l.npar);
     c->launches += 2;
 }
 static void unpack_2row(gfc_ctx *c) {
     const Lat &l = c->lat;
     dim3 gu((l.vh + 255) / 256, 3 * l.npar), gg((l.vh + 255) / 256, l.npar);
-    k_unpack2<<<gu, 256, 0, c->s>>>(c->u64r, c->u, l.vh, 3 * l.npar);
-    k_unpack2<<<gg, 256, 0, c->s>>>(c->g64r, c->g, l.vh, l.npar);
+    launch_early(k_unpack2, gu, 256, 0, c->s, c->u64r, c->u, l.vh, 3 * l.npar);
+    launch_early(k_unpack2, gg, 256, 0, c->s, c->g64r, c->g, l.vh, l.npar);
     c->launches += 2;
 }
 
 // launchers over nblk SoA blocks of `stride` matrices (used by the batch engine)
 void launch_to_f32(const double2 *src, float4 *dst, uint32_t stride, uint32_t nblk, cudaStream_t s) {
-    k_to_f32<<<dim3((stride + 255) / 256, nblk), 256, 0, s>>>(src, dst, stride, nblk);
+    launch_early(k_to_f32, dim3((stride + 255) / 256, nblk), 256, 0, s, src, dst, stride, nblk);
 }
 void launch_identity32(float4 *g, uint32_t stride, uint32_t nblk, cudaStream_t s) {
-    k_identity32<<<dim3((stride + 255) / 256, nblk), 256, 0, s>>>(g, stride, nblk);
+    launch_early(k_identity32, dim3((stride + 255) / 256, nblk), 256, 0, s, g, stride, nblk);
 }
 void launch_pack2(const double2 *src, double2 *dst, uint32_t stride, uint32_t nblk, cudaStream_t s) {
-    k_pack2<<<dim3((stride + 255) / 256, nblk), 256, 0, s>>>(src, dst, stride, nblk);
+    launch_early(k_pack2, dim3((stride + 255) / 256, nblk), 256, 0, s, src, dst, stride, nblk);
 }
 void launch_unpack2(const double2 *src, double2 *dst, uint32_t stride, uint32_t nblk, cudaStream_t s) {
-    k_unpack2<<<dim3((stride + 255) / 256, nblk), 256, 0, s>>>(src, dst, stride, nblk);
+    launch_early(k_unpack2, dim3((stride + 255) / 256, nblk), 256, 0, s, src, dst, stride, nblk);
 }
 
 int halfsweeps_fast64(gfc_ctx *c, int first, int n, double omega, unsigned hits) {
@@ -596,7 +606,7 @@ static void launch_reunit(gfc_ctx *c, typename S::V *base, uint32_t nblk, unsign
     const uint32_t vsh = l.vs >> 1;
     const uint32_t begin = (uint32_t)t0 * vsh, count = nsl < 0 ? l.vh : (uint32_t)nsl * vsh;
     dim3 grid((count + 255) / 256, nblk);
-    k_reunit_fast<S><<<grid, 256, 0, c->s>>>(base, l.vh, nblk, begin, count, stop, c->dstatus);
+    launch_early(k_reunit_fast<S>, grid, 256, 0, c->s, base, l.vh, nblk, begin, count, stop, c->dstatus);
     c->launches++;
 }
 
@@ -615,6 +625,7 @@ __global__ void __launch_bounds__(LEX_BLOCK, 11) k_sweep_lex_fast(double2 *__res
                                                                  Lat l, int sweep, int level, double omega,
                                                                  unsigned hits, const unsigned *stop) {
     extern __shared__ __align__(16) unsigned char lex_stage[];
+    grid_wait();
     if (stop && *(volatile const unsigned *)stop) return;
     uint32_t L;
     if (!odd_parity_site(l, sweep & 1, blockIdx.x * LEX_BLOCK + threadIdx.x, L)) return;
@@ -633,7 +644,7 @@ static void launch_halfsweep_lex_fast(gfc_ctx *c, int sweep, double omega, unsig
     smem_attr_once(done, k_sweep_lex_fast, bytes);
     const unsigned blocks = (unsigned)((l.v / 2 + 1 + LEX_BLOCK - 1) / LEX_BLOCK);
     for (int level = 0; level < 4; level++)
-        k_sweep_lex_fast<<<blocks, LEX_BLOCK, bytes, c->s>>>(c->u64r, c->g64r, l, sweep, level, omega, hits, stop);
+        launch_early(k_sweep_lex_fast, blocks, LEX_BLOCK, bytes, c->s, c->u64r, c->g64r, l, sweep, level, omega, hits, stop);
     c->launches += 4;
 }
 
@@ -642,6 +653,7 @@ static void launch_halfsweep_lex_fast(gfc_ctx *c, int sweep, double omega, unsig
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_e2_lex_fast(const double2 *__restrict__ u, Lat l,
                                                        double *__restrict__ part, const unsigned *stop) {
+    grid_wait();
     if (stop && *(volatile const unsigned *)stop) return;
     __shared__ double sh[2][BLOCK / 32];
     const uint32_t t = blockIdx.y;
@@ -662,7 +674,7 @@ __global__ void __launch_bounds__(BLOCK) k_e2_lex_fast(const double2 *__restrict
 static void launch_e2_lex_fast(gfc_ctx *c, const unsigned *stop) {
     const Lat &l = c->lat;
     const int nbx = obs_blocks_per_slice(l);
-    k_e2_lex_fast<128><<<dim3(nbx, l.nt), 128, 0, c->s>>>(c->u64r, l, c->part, stop);
+    launch_early(k_e2_lex_fast<128>, dim3(nbx, l.nt), 128, 0, c->s, c->u64r, l, c->part, stop);
     launch_finalize2(c->part, l, nbx, c->dres, c->s, stop);
     c->launches += 2;
 }
@@ -1000,8 +1012,8 @@ int fix_mixed(gfc_ctx *c, const gfc_params *p, const gfc_options *o, gfc_report 
     const int maxs = (int)p->max_sweeps_to_fix, K = o->fp32_refresh > 0 ? o->fp32_refresh : 0;
     int done = 0, below = -1;
     bool rebuilt = false;
-    k_to_f32<<<gu, 256, 0, c->s>>>(c->u, (float4 *)c->u32, l.vh, 3 * l.npar);
-    k_identity32<<<gg, 256, 0, c->s>>>((float4 *)c->g32, l.vh, l.npar);
+    launch_early(k_to_f32, gu, 256, 0, c->s, c->u, (float4 *)c->u32, l.vh, 3 * l.npar);
+    launch_early(k_identity32, gg, 256, 0, c->s, (float4 *)c->g32, l.vh, l.npar);
     c->launches += 2;
     // FP32 bulk, in pieces of fp32_refresh half-sweeps when refreshing.  Without
     // refreshing, the FP32 links and G are reunitarised every min(reunit, 50)
@@ -1018,8 +1030,8 @@ int fix_mixed(gfc_ctx *c, const gfc_params *p, const gfc_options *o, gfc_report 
         if (below >= 0 || !K || done >= maxs) break;
         // refresh: G = G32 G in FP64 (projected) and the FP32 G back to the identity,
         // then the FP32 links rounded from G U0 G^dagger computed in FP64
-        k_compose_gt<<<gg, 256, 0, c->s>>>((float4 *)c->g32, c->g, l.vh, 1);
-        k_regauge<S32><<<gs, 128, 0, c->s>>>(U0, c->g, (float4 *)c->u32, l);
+        launch_early(k_compose_gt, gg, 256, 0, c->s, (float4 *)c->g32, c->g, l.vh, 1);
+        launch_early(k_regauge<S32>, gs, 128, 0, c->s, U0, c->g, (float4 *)c->u32, l);
         c->launches += 2;
         rebuilt = true;
     }
@@ -1043,12 +1055,12 @@ int fix_mixed(gfc_ctx *c, const gfc_params *p, const gfc_options *o, gfc_report 
     if (o->warm_start || K) {
         // G = G1 G0: G1 of the FP32 phase times the starting G0 (a warm start's, or
         // the one accumulated by the refreshes)
-        k_compose_gt<<<gg, 256, 0, c->s>>>((float4 *)c->g32, c->g, l.vh, 0);
+        launch_early(k_compose_gt, gg, 256, 0, c->s, (float4 *)c->g32, c->g, l.vh, 0);
     } else {
-        k_to_f64<<<gg, 256, 0, c->s>>>((const float4 *)c->g32, c->g, l.vh, l.npar);
+        launch_early(k_to_f64, gg, 256, 0, c->s, (const float4 *)c->g32, c->g, l.vh, l.npar);
     }
-    k_regauge<S64R><<<gs, 128, 0, c->s>>>(U0, c->g, c->u64r, l);
-    k_pack2<<<gg, 256, 0, c->s>>>(c->g, c->g64r, l.vh, l.npar);
+    launch_early(k_regauge<S64R>, gs, 128, 0, c->s, U0, c->g, c->u64r, l);
+    launch_early(k_pack2, gg, 256, 0, c->s, c->g, c->g64r, l.vh, l.npar);
     c->launches += 3;
     // FP64 refinement
     unsigned reunit64 = o->refine_reunit ? o->refine_reunit : p->sweeps_to_reunitarization;
@@ -1152,8 +1164,8 @@ extern "C" int gfc_ctx_autotune(gfc_ctx *c, int which, double *times_out) {
     }
     if ((which & 4) && c->u32 && c->g32) {
         dim3 gu((l.vh + 255) / 256, 3 * l.npar), gg((l.vh + 255) / 256, l.npar);
-        k_to_f32<<<gu, 256, 0, c->s>>>(c->u, (float4 *)c->u32, l.vh, 3 * l.npar);
-        k_identity32<<<gg, 256, 0, c->s>>>((float4 *)c->g32, l.vh, l.npar);
+        launch_early(k_to_f32, gu, 256, 0, c->s, c->u, (float4 *)c->u32, l.vh, 3 * l.npar);
+        launch_early(k_identity32, gg, 256, 0, c->s, (float4 *)c->g32, l.vh, l.npar);
         double best = 1e30;
         for (int v = 0; v < kNumAll; v++) {
             double t = timed([&](int k) {

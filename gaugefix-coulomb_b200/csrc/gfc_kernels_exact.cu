@@ -70,6 +70,7 @@ template <int BLOCK, int MINB>
 __global__ void __launch_bounds__(BLOCK, MINB) k_sweep_exact(double2 *__restrict__ u, double2 *__restrict__ g,
                                                              Lat l, int par, double omega, unsigned hits,
                                                              const unsigned *stop) {
+    grid_wait();
     if (stop && *(volatile const unsigned *)stop) return;
     uint32_t i = blockIdx.x * BLOCK + threadIdx.x;
     if (i >= l.vh) return;
@@ -158,6 +159,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_sweep_exact_staged(double2 *__r
                                                                     double omega, unsigned hits,
                                                                     const unsigned *stop) {
     extern __shared__ __align__(16) unsigned char exact_stage[];
+    grid_wait();
     if (stop && *(volatile const unsigned *)stop) return;
     uint32_t i = blockIdx.x * BLOCK + threadIdx.x;
     if (i >= l.vh) return;
@@ -173,7 +175,7 @@ static void launch_exact_staged(const Lat &l, double2 *u, double2 *g, int par, d
     auto kern = k_sweep_exact_staged<BLOCK, MINB>;
     static std::atomic<unsigned long long> done{0};
     smem_attr_once(done, kern, bytes);
-    kern<<<(l.vh + BLOCK - 1) / BLOCK, BLOCK, bytes, s>>>(u, g, l, par, omega, hits, stop);
+    launch_early(kern, (l.vh + BLOCK - 1) / BLOCK, BLOCK, bytes, s, u, g, l, par, omega, hits, stop);
 }
 
 // Odd ns: same-parity sites meet across the periodic boundary, so the updates of a
@@ -197,6 +199,7 @@ __global__ void __launch_bounds__(LEVEL_BLOCK, 8) k_sweep_exact_level(double2 *_
                                                                      int level, double omega, unsigned hits,
                                                                      const unsigned *stop) {
     extern __shared__ __align__(16) unsigned char level_stage[];
+    grid_wait();
     if (stop && *(volatile const unsigned *)stop) return;
     uint32_t L;
     // BLACKRED_SWEEP (gauge_fixing.c:42): parity (x + y + z + t) & 1 = sweep & 1
@@ -222,7 +225,7 @@ int launch_sweep_exact(double2 *u, double2 *g, const Lat &l, int sweep, double o
         int par = sweep & 1;  // BLACKRED_SWEEP: even sites on even sweeps (gauge_fixing.c:42)
         switch (shape) {
             case 1:
-                k_sweep_exact<128, 3><<<(l.vh + 127) / 128, 128, 0, s>>>(u, g, l, par, omega, hits, stop);
+                launch_early(k_sweep_exact<128, 3>, (l.vh + 127) / 128, 128, 0, s, u, g, l, par, omega, hits, stop);
                 break;
             case 2:   // 27 KiB per CTA, 8 CTAs per SM
                 launch_exact_staged<32, 8>(l, u, g, par, omega, hits, s, stop);
@@ -235,7 +238,7 @@ int launch_sweep_exact(double2 *u, double2 *g, const Lat &l, int sweep, double o
                 break;
 
             default:
-                k_sweep_exact<128, 1><<<(l.vh + 127) / 128, 128, 0, s>>>(u, g, l, par, omega, hits, stop);
+                launch_early(k_sweep_exact<128, 1>, (l.vh + 127) / 128, 128, 0, s, u, g, l, par, omega, hits, stop);
                 break;
         }
     } else {
@@ -245,7 +248,7 @@ int launch_sweep_exact(double2 *u, double2 *g, const Lat &l, int sweep, double o
         smem_attr_once(done, k_sweep_exact_level, bytes);
         const unsigned blocks = (unsigned)((l.v / 2 + 1 + LEVEL_BLOCK - 1) / LEVEL_BLOCK);
         for (int level = 0; level < 4; level++)
-            k_sweep_exact_level<<<blocks, LEVEL_BLOCK, bytes, s>>>(u, g, l, sweep, level, omega, hits, stop);
+            launch_early(k_sweep_exact_level, blocks, LEVEL_BLOCK, bytes, s, u, g, l, sweep, level, omega, hits, stop);
         return 4;
     }
     return 1;
@@ -256,6 +259,7 @@ int launch_sweep_exact(double2 *u, double2 *g, const Lat &l, int sweep, double o
 // SoA matrices laid out as [c][stride] blocks starting at base + k*9*stride.
 __global__ void k_reunitarize(double2 *__restrict__ base, uint32_t stride, uint32_t nblk,
                               unsigned *__restrict__ status) {
+    grid_wait();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t k = blockIdx.y;
     if (i >= stride || k >= nblk) return;
@@ -269,10 +273,11 @@ __global__ void k_reunitarize(double2 *__restrict__ base, uint32_t stride, uint3
 
 void launch_reunitarize(double2 *base, uint32_t stride, uint32_t nblk, unsigned *status, cudaStream_t s) {
     dim3 grid((stride + 255) / 256, nblk);
-    k_reunitarize<<<grid, 256, 0, s>>>(base, stride, nblk, status);
+    launch_early(k_reunitarize, grid, 256, 0, s, base, stride, nblk, status);
 }
 
 __global__ void k_identity(double2 *__restrict__ g, uint32_t n) {
+    grid_wait();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
 #pragma unroll
@@ -282,7 +287,7 @@ __global__ void k_identity(double2 *__restrict__ g, uint32_t n) {
 // G is npar blocks of [9][vh]; treat it as one [9][npar*vh] run per block
 void launch_identity(double2 *g, const Lat &l, cudaStream_t s) {
     for (int p = 0; p < l.npar; p++)
-        k_identity<<<(l.vh + 255) / 256, 256, 0, s>>>(g + (size_t)p * 9 * l.vh, l.vh);
+        launch_early(k_identity, (l.vh + 255) / 256, 256, 0, s, g + (size_t)p * 9 * l.vh, l.vh);
 }
 
 // ------------------------------------------------------------- observables --
@@ -393,6 +398,7 @@ __device__ __forceinline__ void block_sum(double (&v)[NQ]) {
 // registers), so three blocks (12 warps) fit on an SM where one 256-thread block did
 __global__ void __launch_bounds__(128) k_obs_partials(const double2 *__restrict__ u, Lat l,
                                                       double *__restrict__ part, const unsigned *stop) {
+    grid_wait();
     if (stop && *(volatile const unsigned *)stop) return;
     const uint32_t t = blockIdx.y;
     const uint32_t vsh = l.cb ? l.vs / 2 : l.vs;  // slots of one parity per slice
@@ -423,6 +429,7 @@ __global__ void __launch_bounds__(128) k_obs_partials(const double2 *__restrict_
 // F density: Re Tr of the 3 spatial links at a site (calculateF, gauge_fixing.c:289-337)
 __global__ void __launch_bounds__(256) k_functional_partials(const double2 *__restrict__ u, Lat l,
                                                              double *__restrict__ part) {
+    grid_wait();
     const uint32_t t = blockIdx.y;
     const uint32_t vsh = l.cb ? l.vs / 2 : l.vs;
     const uint32_t n = vsh * l.npar;
@@ -444,6 +451,7 @@ __global__ void __launch_bounds__(256) k_functional_partials(const double2 *__re
 // out[q] = total, slice_out[t*nq + q] = per slice (optional).
 __global__ void k_finalize(const double *__restrict__ part, int nt, int nbx, int nq, double *__restrict__ out,
                            double *__restrict__ slice_out, const unsigned *stop) {
+    grid_wait();
     if (stop && *(volatile const unsigned *)stop) return;
     __shared__ double acc[4][256];
     for (int q = 0; q < nq; q++) acc[q][threadIdx.x] = 0.0;
@@ -478,14 +486,14 @@ int obs_blocks_per_slice(const Lat &l) {
 
 // sums of nbx per-block (e2, theta) partials per timeslice into out[0..1]
 void launch_finalize2(const double *part, const Lat &l, int nbx, double *out, cudaStream_t s, const unsigned *stop) {
-    k_finalize<<<1, 256, 0, s>>>(part, l.nt, nbx, 2, out, nullptr, stop);
+    launch_early(k_finalize, 1, 256, 0, s, part, l.nt, nbx, 2, out, nullptr, stop);
 }
 
 void launch_obs(const double2 *u, const Lat &l, double *part, double *out, double *slice_out, cudaStream_t s,
                 const unsigned *stop) {
     int nbx = obs_blocks_per_slice(l);
-    k_obs_partials<<<dim3(nbx, l.nt), 128, 0, s>>>(u, l, part, stop);
-    k_finalize<<<1, 256, 0, s>>>(part, l.nt, nbx, 2, out, slice_out, stop);
+    launch_early(k_obs_partials, dim3(nbx, l.nt), 128, 0, s, u, l, part, stop);
+    launch_early(k_finalize, 1, 256, 0, s, part, l.nt, nbx, 2, out, slice_out, stop);
 }
 
 // After the observables of half-sweep `sweep`: the proxy (e2 = out[0] / V, or theta =
@@ -493,6 +501,7 @@ void launch_obs(const double2 *u, const Lat &l, double *part, double *out, doubl
 // sweep, once; later sweep and observables launches of the stream then do nothing.
 __global__ void k_exact_check(const double *__restrict__ out, double v, int theta, double tol, int sweep,
                               unsigned *stop) {
+    grid_wait();
     if (threadIdx.x || blockIdx.x || *(volatile unsigned *)stop) return;
     const double res = theta ? out[1] / (3.0 * v) : out[0] / v;
     if (res <= tol) *stop = (unsigned)sweep;
@@ -500,13 +509,13 @@ __global__ void k_exact_check(const double *__restrict__ out, double v, int thet
 
 void launch_exact_check(const double *out, const Lat &l, int theta, double tol, int sweep, unsigned *stop,
                         cudaStream_t s) {
-    k_exact_check<<<1, 32, 0, s>>>(out, (double)l.v, theta, tol, sweep, stop);
+    launch_early(k_exact_check, 1, 32, 0, s, out, (double)l.v, theta, tol, sweep, stop);
 }
 
 void launch_functional(const double2 *u, const Lat &l, double *part, double *out, cudaStream_t s) {
     int nbx = obs_blocks_per_slice(l);
-    k_functional_partials<<<dim3(nbx, l.nt), 256, 0, s>>>(u, l, part);
-    k_finalize<<<1, 256, 0, s>>>(part, l.nt, nbx, 1, out, nullptr, nullptr);
+    launch_early(k_functional_partials, dim3(nbx, l.nt), 256, 0, s, u, l, part);
+    launch_early(k_finalize, 1, 256, 0, s, part, l.nt, nbx, 1, out, nullptr, nullptr);
 }
 
 }  // namespace gfc

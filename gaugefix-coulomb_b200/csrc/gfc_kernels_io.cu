@@ -153,6 +153,7 @@ __device__ __forceinline__ void gug(const M3 &gx, const M3 &uu, const M3 &gy, M3
 }
 
 __global__ void k_temporal_transform(double2 *__restrict__ ut, const double2 *__restrict__ g, Lat l) {
+    grid_wait();
     uint32_t L = blockIdx.x * blockDim.x + threadIdx.x;
     if (L >= l.v) return;
     Coord c = coord_lex(l, L);
@@ -166,11 +167,12 @@ __global__ void k_temporal_transform(double2 *__restrict__ ut, const double2 *__
 }
 
 void launch_temporal_transform(double2 *ut, const double2 *g, const Lat &l, cudaStream_t s) {
-    k_temporal_transform<<<(l.v + 127) / 128, 128, 0, s>>>(ut, g, l);
+    launch_early(k_temporal_transform, (l.v + 127) / 128, 128, 0, s, ut, g, l);
 }
 
 __global__ void k_apply_gt_spatial(double2 *__restrict__ u, const double2 *__restrict__ u0,
                                    const double2 *__restrict__ g, Lat l) {
+    grid_wait();
     uint32_t L = blockIdx.x * blockDim.x + threadIdx.x;
     if (L >= l.v) return;
     Coord c = coord_lex(l, L);
@@ -210,6 +212,7 @@ __device__ __forceinline__ void xvuwdag(const M3 &v, const M3 &u, const M3 &w, M
 // Each thread reads and writes only the links of its own site.
 __global__ void k_apply_gt(double2 *__restrict__ u, double2 *__restrict__ ut, const double2 *__restrict__ g,
                            Lat l, int temporal) {
+    grid_wait();
     uint32_t L = blockIdx.x * blockDim.x + threadIdx.x;
     if (L >= l.v) return;
     Coord c = coord_lex(l, L);
@@ -234,11 +237,11 @@ __global__ void k_apply_gt(double2 *__restrict__ u, double2 *__restrict__ ut, co
 }
 
 void launch_apply_gt(double2 *u, double2 *ut, const double2 *g, const Lat &l, int temporal, cudaStream_t s) {
-    k_apply_gt<<<(l.v + 127) / 128, 128, 0, s>>>(u, ut, g, l, temporal);
+    launch_early(k_apply_gt, (l.v + 127) / 128, 128, 0, s, u, ut, g, l, temporal);
 }
 
 void launch_apply_gt_spatial(double2 *u, const double2 *u0, const double2 *g, const Lat &l, cudaStream_t s) {
-    k_apply_gt_spatial<<<(l.v + 127) / 128, 128, 0, s>>>(u, u0, g, l);
+    launch_early(k_apply_gt_spatial, (l.v + 127) / 128, 128, 0, s, u, u0, g, l);
 }
 
 // ---------------------------------------------------------------- plaquette --
@@ -299,6 +302,7 @@ __device__ __forceinline__ void block_sum2(double &a, double &b) {
 __global__ void __launch_bounds__(256) k_plaquette_partials(const double2 *__restrict__ u,
                                                             const double2 *__restrict__ ut, Lat l,
                                                             double *__restrict__ part) {
+    grid_wait();
     const uint32_t t = blockIdx.y;
     double sp = 0.0, tp = 0.0;
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < l.vs; k += gridDim.x * blockDim.x) {
@@ -317,6 +321,7 @@ __global__ void __launch_bounds__(256) k_plaquette_partials(const double2 *__res
 }
 
 __global__ void k_finalize2(const double *__restrict__ part, int nt, int nbx, double *__restrict__ out) {
+    grid_wait();
     __shared__ double acc[2][256];
     acc[0][threadIdx.x] = 0.0;
     acc[1][threadIdx.x] = 0.0;
@@ -343,8 +348,8 @@ __global__ void k_finalize2(const double *__restrict__ part, int nt, int nbx, do
 void launch_plaquette(const double2 *u, const double2 *ut, const Lat &l, double *part, double *out,
                       cudaStream_t s) {
     int nbx = obs_blocks_per_slice(l);
-    k_plaquette_partials<<<dim3(nbx, l.nt), 256, 0, s>>>(u, ut, l, part);
-    k_finalize2<<<1, 256, 0, s>>>(part, l.nt, nbx, out);
+    launch_early(k_plaquette_partials, dim3(nbx, l.nt), 256, 0, s, u, ut, l, part);
+    launch_early(k_finalize2, 1, 256, 0, s, part, l.nt, nbx, out);
 }
 
 }  // namespace gfc
