@@ -107,20 +107,42 @@ __host__ __device__ __forceinline__ uint32_t back_L(const Lat &l, const Coord &c
     if (d == 1) return c.y ? c.L - ns : c.L + (ns - 1) * ns;
     return c.x ? c.L - 1 : c.L + (ns - 1);
 }
-// The k-th site of parity p = (x + y + z + t) & 1 in lexicographic order, odd ns: row
-// R (of ns sites along x) has row parity R & 1 (ns is odd, so R = y + ns z + ns^2 t has
-// the parity of y + z + t), so the sites of parity p in a row are x = p ^ (R & 1), +2,
-// ...; a pair of rows holds exactly ns of them, (ns + 1) / 2 in its first row when
-// p = 0, (ns - 1) / 2 when p = 1.  False past the last one.
-__device__ __forceinline__ bool odd_parity_site(const Lat &l, int p, uint32_t k, uint32_t &L) {
-    const uint32_t ns = (uint32_t)l.ns;
-    const uint32_t a = p ? (ns - 1) >> 1 : (ns + 1) >> 1;   // in the first (even) row of a pair
-    const uint32_t pair = k / ns, rem = k - pair * ns;
-    const uint32_t R = rem < a ? 2 * pair : 2 * pair + 1;
-    const uint32_t j = rem < a ? rem : rem - a;
-    const uint32_t x = 2 * j + ((uint32_t)p ^ (R & 1u));
-    L = x + ns * R;
-    return R < (uint32_t)l.ns * (uint32_t)l.ns * (uint32_t)l.nt;
+// The sites of a boundary level of one parity, odd ns.  Level v has the sites with v
+// coordinates equal to e = ns - 1 and the others in [0, e): e is even, so those others
+// run over an even lattice of 3 - v dimensions, half of whose sites have either parity,
+// and the level's sites are numbered without gaps: level 0 e^3 / 2 sites, level 1 three
+// faces of e^2 / 2, level 2 three edges of e / 2, level 3 one corner (on timeslices of
+// its parity).  A launch over a level has a full warp of its sites for every 32, where
+// one that tests every site of the parity for the level has mostly idle ones.
+__host__ __device__ __forceinline__ uint32_t odd_level_count(const Lat &l, int level) {
+    const uint32_t e = (uint32_t)l.ns - 1;
+    return level == 0 ? e * e * e / 2 : level == 1 ? 3 * (e * e / 2) : level == 2 ? 3 * (e / 2) : 1u;
+}
+// site j < odd_level_count of parity p = (x + y + z + t) & 1 on timeslice t: its index
+// inside the timeslice; false for a corner of the other parity
+__host__ __device__ __forceinline__ bool odd_level_site(const Lat &l, int p, uint32_t t, int level, uint32_t j,
+                                                        uint32_t &off) {
+    const uint32_t ns = (uint32_t)l.ns, e = ns - 1;
+    const uint32_t q = ((uint32_t)p ^ t) & 1u;
+    if (level == 3) {
+        off = (e * ns + e) * ns + e;
+        return q == 0;
+    }
+    if (level == 2) {
+        const uint32_t f = j / (e / 2), c = 2 * (j - f * (e / 2)) + q;
+        off = f == 0 ? (e * ns + e) * ns + c : f == 1 ? (e * ns + c) * ns + e : (c * ns + e) * ns + e;
+        return true;
+    }
+    if (level == 1) {
+        const uint32_t n = e * e / 2, f = j / n, r = 2 * (j - f * n);
+        const uint32_t b = r / e, a = r - b * e + (q ^ (b & 1u));
+        off = f == 0 ? (e * ns + b) * ns + a : f == 1 ? (b * ns + e) * ns + a : (b * ns + a) * ns + e;
+        return true;
+    }
+    const uint32_t r = 2 * j, R = r / e, z = R / e, y = R - z * e;
+    const uint32_t x = r - R * e + (q ^ ((y + z) & 1u));
+    off = (z * ns + y) * ns + x;
+    return true;
 }
 
 __host__ __device__ __forceinline__ uint32_t fwd_L(const Lat &l, const Coord &c, int d) {

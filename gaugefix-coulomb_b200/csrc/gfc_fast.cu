@@ -616,10 +616,9 @@ static void print_res(int sweep, double res) { printf("Sweeps: %8d.\t residue: %
 // Odd ns with the fast arithmetic (FP64 on two stored rows, lexicographic layout): a
 // half-sweep is the four boundary-level launches of the exact path (the sequential
 // sweep's order between every pair of sites that share a link, see
-// k_sweep_exact_level), each thread taking a site of the half-sweep's parity
-// (odd_parity_site) and updating it if it has the launch's level.  e2 is measured by
-// a separate pass over the state a half-sweep leaves: a site's post-update w is not
-// final while a later level updates a neighbour.
+// k_sweep_exact_level) over the level's sites of the half-sweep's parity
+// (odd_level_site).  e2 is measured by a separate pass over the state a half-sweep
+// leaves: a site's post-update w is not final while a later level updates a neighbour.
 constexpr int LEX_BLOCK = 32;
 __global__ void __launch_bounds__(LEX_BLOCK, 11) k_sweep_lex_fast(double2 *__restrict__ u, double2 *__restrict__ g,
                                                                  Lat l, int sweep, int level, double omega,
@@ -627,13 +626,11 @@ __global__ void __launch_bounds__(LEX_BLOCK, 11) k_sweep_lex_fast(double2 *__res
     extern __shared__ __align__(16) unsigned char lex_stage[];
     grid_wait();
     if (stop && *(volatile const unsigned *)stop) return;
-    uint32_t L;
-    if (!odd_parity_site(l, sweep & 1, blockIdx.x * LEX_BLOCK + threadIdx.x, L)) return;
-    const Coord c = coord_lex(l, L);
-    const uint32_t e = (uint32_t)l.ns - 1;
-    if ((int)(c.x == e) + (int)(c.y == e) + (int)(c.z == e) != level) return;
+    const uint32_t n = odd_level_count(l, level), k = blockIdx.x * LEX_BLOCK + threadIdx.x, t = k / n;
+    uint32_t off;
+    if (t >= (uint32_t)l.nt || !odd_level_site(l, sweep & 1, t, level, k - t * n, off)) return;
     double pre = 0.0, post = 0.0;
-    fast_site_staged<S64R, LEX_BLOCK, false, 6, false>(u, g, l, 0, L, omega, hits, 0, pre, post,
+    fast_site_staged<S64R, LEX_BLOCK, false, 6, false>(u, g, l, 0, t * l.vs + off, omega, hits, 0, pre, post,
                                                        (double2 *)lex_stage);
 }
 
@@ -642,9 +639,8 @@ static void launch_halfsweep_lex_fast(gfc_ctx *c, int sweep, double omega, unsig
     constexpr size_t bytes = (size_t)6 * S64R::NS * LEX_BLOCK * sizeof(double2);
     static std::atomic<unsigned long long> done{0};
     smem_attr_once(done, k_sweep_lex_fast, bytes);
-    const unsigned blocks = (unsigned)((l.v / 2 + 1 + LEX_BLOCK - 1) / LEX_BLOCK);
     for (int level = 0; level < 4; level++)
-        launch_early(k_sweep_lex_fast, blocks, LEX_BLOCK, bytes, c->s, c->u64r, c->g64r, l, sweep, level, omega, hits, stop);
+        launch_early(k_sweep_lex_fast, (odd_level_count(l, level) * l.nt + LEX_BLOCK - 1) / LEX_BLOCK, LEX_BLOCK, bytes, c->s, c->u64r, c->g64r, l, sweep, level, omega, hits, stop);
     c->launches += 4;
 }
 
