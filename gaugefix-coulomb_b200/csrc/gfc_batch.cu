@@ -38,8 +38,8 @@
 namespace gfc {
 
 enum : int { SS_EMPTY = 0, SS_FP32 = 1, SS_PEND = 2, SS_FP64 = 3, SS_DONE = 4, SS_VERIFY = 5, SS_LEX = 6 };
-// SS_LEX: a timeslice of an odd-ns lattice, FP64 on two stored rows in the
-// lexicographic layout.  Same-parity sites meet across the periodic boundary there,
+// SS_LEX: a timeslice of an odd-ns lattice, FP64 on two stored rows in the odd-ns
+// working layout (odd_slot).  Same-parity sites meet across the periodic boundary there,
 // so a half-sweep runs as four launches over the boundary levels (the number of
 // coordinates equal to ns - 1), which keeps the order of the sequential z, y, x
 // sweep between every pair of sites that share a link; e2 is measured by a separate
@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(32) k_bmeasure_lex(BState b) {
 #pragma unroll 1
             for (int q = 0; q < BPIECES; q++) {
                 const uint32_t off = (uint32_t)item.y * BCHUNK + (uint32_t)q * 32 + lane;
-                double v = off < l.vs ? measure_site<S64R, false>(sl.u64r, l, 0, (uint32_t)t * l.vs + off) : 0.0;
+                double v = off < l.vs ? measure_site<S64R, false>(sl.u64r, l, 0, odd_site(l.ns, (uint32_t)t * l.vs + off)) : 0.0;
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
                 if (lane == 0) {
@@ -1162,18 +1162,18 @@ extern "C" int gfc_batch_activate(gfc_batch *b, int slot, int precision) {
     launch_identity(sl.g, l, b->s);
     int st;
     if (!l.cb) {
-        // odd ns: FP64 on two stored rows in the lexicographic layout, whatever the
+        // odd ns: FP64 on two stored rows in the odd_slot order, whatever the
         // precision asked for (the FP32 phase and its switch need the checkerboard)
-        launch_pack2(sl.u, sl.u64r, l.vh, 3 * l.npar, b->s);
-        launch_pack2(sl.g, sl.g64r, l.vh, l.npar, b->s);
+        launch_pack2(sl.u, sl.u64r, l.vh, 3 * l.npar, (uint32_t)l.ns, b->s);
+        launch_pack2(sl.g, sl.g64r, l.vh, l.npar, (uint32_t)l.ns, b->s);
         st = SS_LEX;
     } else if (precision == GFC_PREC_MIXED) {
         launch_to_f32(sl.u, sl.u32, l.vh, 3 * l.npar, b->s);
         launch_identity32(sl.g32, l.vh, l.npar, b->s);
         st = SS_FP32;
     } else {
-        launch_pack2(sl.u, sl.u64r, l.vh, 3 * l.npar, b->s);
-        launch_pack2(sl.g, sl.g64r, l.vh, l.npar, b->s);
+        launch_pack2(sl.u, sl.u64r, l.vh, 3 * l.npar, 0, b->s);
+        launch_pack2(sl.g, sl.g64r, l.vh, l.npar, 0, b->s);
         st = SS_FP64;
     }
     BState bs{};
@@ -1402,8 +1402,8 @@ extern "C" int gfc_batch_finalize(gfc_batch *b, int slot, gfc_report *r) {
     const BSlot &sl = b->hs[slot];
     const Lat &l = sl.l;
     launch_early(k_set_state, (l.nt + 127) / 128, 128, 0, b->s, b->state, slot * b->max_nt, l.nt, SS_DONE);
-    launch_unpack2(sl.u64r, sl.u, l.vh, 3 * l.npar, b->s);
-    launch_unpack2(sl.g64r, sl.g, l.vh, l.npar, b->s);
+    launch_unpack2(sl.u64r, sl.u, l.vh, 3 * l.npar, l.cb ? 0u : (uint32_t)l.ns, b->s);
+    launch_unpack2(sl.g64r, sl.g, l.vh, l.npar, l.cb ? 0u : (uint32_t)l.ns, b->s);
     launch_reunitarize(sl.u, l.vh, 3 * l.npar, b->status, b->s);
     launch_reunitarize(sl.g, l.vh, l.npar, b->status, b->s);
     launch_temporal_transform(sl.ut, sl.g, l, b->s);

@@ -107,6 +107,19 @@ __host__ __device__ __forceinline__ uint32_t back_L(const Lat &l, const Coord &c
     if (d == 1) return c.y ? c.L - ns : c.L + (ns - 1) * ns;
     return c.x ? c.L - 1 : c.L + (ns - 1);
 }
+// Odd ns, two-row working fields: within a row of ns sites the (ns + 1) / 2 sites of even
+// x come first, then those of odd x, so the sites of one parity in a row (all of one x
+// parity) are neighbours and a warp uses whole sectors; in lexicographic order every
+// other site of a sector is the other parity's.  Slot of the site with lexicographic
+// index L and coordinate x, and the site of a slot.
+__host__ __device__ __forceinline__ uint32_t odd_slot(const Lat &l, uint32_t L, uint32_t x) {
+    return L - x + (x >> 1) + ((x & 1u) ? ((uint32_t)l.ns + 1) >> 1 : 0u);
+}
+__host__ __device__ __forceinline__ uint32_t odd_site(uint32_t ns, uint32_t i) {
+    const uint32_t s = i % ns, h = (ns + 1) >> 1;
+    return i - s + (s < h ? 2 * s : 2 * (s - h) + 1);
+}
+
 // The sites of a boundary level of one parity, odd ns.  Level v has the sites with v
 // coordinates equal to e = ns - 1 and the others in [0, e): e is even, so those others
 // run over an even lattice of 3 - v dimensions, half of whose sites have either parity,

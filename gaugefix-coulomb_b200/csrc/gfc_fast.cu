@@ -274,25 +274,28 @@ __global__ void k_to_f64(const float4 *__restrict__ src, double2 *__restrict__ d
     for (int e = 0; e < 9; e++) q[(size_t)e * stride] = m.e[e];
 }
 
-// FP64 full SoA ([9][stride] per block) -> FP64 two-row SoA ([6][stride])
-__global__ void k_pack2(const double2 *__restrict__ src, double2 *__restrict__ dst, uint32_t stride, uint32_t nblk) {
+// FP64 full SoA ([9][stride] per block) -> FP64 two-row SoA ([6][stride]); odd_ns != 0:
+// the two-row field in the odd-ns working order (odd_slot)
+__global__ void k_pack2(const double2 *__restrict__ src, double2 *__restrict__ dst, uint32_t stride, uint32_t nblk,
+                        uint32_t odd_ns) {
     grid_wait();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
     if (i >= stride || k >= nblk) return;
-    const double2 *p = src + (size_t)k * 9 * stride + i;
+    const double2 *p = src + (size_t)k * 9 * stride + (odd_ns ? odd_site(odd_ns, i) : i);
     double2 *q = dst + (size_t)k * 6 * stride + i;
 #pragma unroll
     for (int e = 0; e < 6; e++) q[(size_t)e * stride] = p[(size_t)e * stride];
 }
 
 // FP64 two-row -> full, row 2 = conj(row0 x row1)
-__global__ void k_unpack2(const double2 *__restrict__ src, double2 *__restrict__ dst, uint32_t stride, uint32_t nblk) {
+__global__ void k_unpack2(const double2 *__restrict__ src, double2 *__restrict__ dst, uint32_t stride, uint32_t nblk,
+                          uint32_t odd_ns) {
     grid_wait();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
     if (i >= stride || k >= nblk) return;
     Mt<double> m;
     S64R::load(src + (size_t)k * 6 * stride + i, stride, m);
-    S64::store(dst + (size_t)k * 9 * stride + i, stride, m);
+    S64::store(dst + (size_t)k * 9 * stride + (odd_ns ? odd_site(odd_ns, i) : i), stride, m);
 }
 
 // Slice-blocked sweeping: after a round, e2 after s half-sweeps is
@@ -559,18 +562,19 @@ static int ensure_2row(gfc_ctx *c) {
     if (!c->g64r) GFC_CHECK(cudaMalloc(&c->g64r, (size_t)l.npar * l.vh * 6 * sizeof(double2)));
     return GFC_OK;
 }
+static uint32_t odd_ns_of(const Lat &l) { return l.cb ? 0u : (uint32_t)l.ns; }
 static void pack_2row(gfc_ctx *c) {
     const Lat &l = c->lat;
     dim3 gu((l.vh + 255) / 256, 3 * l.npar), gg((l.vh + 255) / 256, l.npar);
-    launch_early(k_pack2, gu, 256, 0, c->s, c->u, c->u64r, l.vh, 3 * l.npar);
-    launch_early(k_pack2, gg, 256, 0, c->s, c->g, c->g64r, l.vh, l.npar);
+    launch_early(k_pack2, gu, 256, 0, c->s, c->u, c->u64r, l.vh, 3 * l.npar, odd_ns_of(l));
+    launch_early(k_pack2, gg, 256, 0, c->s, c->g, c->g64r, l.vh, l.npar, odd_ns_of(l));
     c->launches += 2;
 }
 static void unpack_2row(gfc_ctx *c) {
     const Lat &l = c->lat;
     dim3 gu((l.vh + 255) / 256, 3 * l.npar), gg((l.vh + 255) / 256, l.npar);
-    launch_early(k_unpack2, gu, 256, 0, c->s, c->u64r, c->u, l.vh, 3 * l.npar);
-    launch_early(k_unpack2, gg, 256, 0, c->s, c->g64r, c->g, l.vh, l.npar);
+    launch_early(k_unpack2, gu, 256, 0, c->s, c->u64r, c->u, l.vh, 3 * l.npar, odd_ns_of(l));
+    launch_early(k_unpack2, gg, 256, 0, c->s, c->g64r, c->g, l.vh, l.npar, odd_ns_of(l));
     c->launches += 2;
 }
 
@@ -581,11 +585,11 @@ void launch_to_f32(const double2 *src, float4 *dst, uint32_t stride, uint32_t nb
 void launch_identity32(float4 *g, uint32_t stride, uint32_t nblk, cudaStream_t s) {
     launch_early(k_identity32, dim3((stride + 255) / 256, nblk), 256, 0, s, g, stride, nblk);
 }
-void launch_pack2(const double2 *src, double2 *dst, uint32_t stride, uint32_t nblk, cudaStream_t s) {
-    launch_early(k_pack2, dim3((stride + 255) / 256, nblk), 256, 0, s, src, dst, stride, nblk);
+void launch_pack2(const double2 *src, double2 *dst, uint32_t stride, uint32_t nblk, uint32_t odd_ns, cudaStream_t s) {
+    launch_early(k_pack2, dim3((stride + 255) / 256, nblk), 256, 0, s, src, dst, stride, nblk, odd_ns);
 }
-void launch_unpack2(const double2 *src, double2 *dst, uint32_t stride, uint32_t nblk, cudaStream_t s) {
-    launch_early(k_unpack2, dim3((stride + 255) / 256, nblk), 256, 0, s, src, dst, stride, nblk);
+void launch_unpack2(const double2 *src, double2 *dst, uint32_t stride, uint32_t nblk, uint32_t odd_ns, cudaStream_t s) {
+    launch_early(k_unpack2, dim3((stride + 255) / 256, nblk), 256, 0, s, src, dst, stride, nblk, odd_ns);
 }
 
 int halfsweeps_fast64(gfc_ctx *c, int first, int n, double omega, unsigned hits) {
@@ -613,7 +617,7 @@ static void launch_reunit(gfc_ctx *c, typename S::V *base, uint32_t nblk, unsign
 static void print_res(int sweep, double res) { printf("Sweeps: %8d.\t residue: %3.2E \n", sweep, res); }
 
 // ----------------------------------------------------------------- odd ns --
-// Odd ns with the fast arithmetic (FP64 on two stored rows, lexicographic layout): a
+// Odd ns with the fast arithmetic (FP64 on two stored rows in the odd_slot order): a
 // half-sweep is the four boundary-level launches of the exact path (the sequential
 // sweep's order between every pair of sites that share a link, see
 // k_sweep_exact_level) over the level's sites of the half-sweep's parity
@@ -644,8 +648,8 @@ static void launch_halfsweep_lex_fast(gfc_ctx *c, int sweep, double omega, unsig
     c->launches += 4;
 }
 
-// e2 and theta partials (theta = e2 / 6 identically) per timeslice of the two-row
-// lexicographic links: grid (nbx, nt), fixed summation order
+// e2 and theta partials (theta = e2 / 6 identically) per timeslice of the two-row links of
+// odd ns, in the order of their slots: grid (nbx, nt), fixed summation order
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_e2_lex_fast(const double2 *__restrict__ u, Lat l,
                                                        double *__restrict__ part, const unsigned *stop) {
@@ -655,7 +659,7 @@ __global__ void __launch_bounds__(BLOCK) k_e2_lex_fast(const double2 *__restrict
     const uint32_t t = blockIdx.y;
     double v[2] = {0.0, 0.0};
     for (uint32_t k = blockIdx.x * BLOCK + threadIdx.x; k < l.vs; k += gridDim.x * BLOCK) {
-        const double e2 = measure_site<S64R, false>(u, l, 0, t * l.vs + k);
+        const double e2 = measure_site<S64R, false>(u, l, 0, odd_site(l.ns, t * l.vs + k));
         v[0] += e2;
         v[1] += 0.5 * e2;   // Re Tr(div A div A^dagger) of the site
     }
@@ -1056,7 +1060,7 @@ int fix_mixed(gfc_ctx *c, const gfc_params *p, const gfc_options *o, gfc_report 
         launch_early(k_to_f64, gg, 256, 0, c->s, (const float4 *)c->g32, c->g, l.vh, l.npar);
     }
     launch_early(k_regauge<S64R>, gs, 128, 0, c->s, U0, c->g, c->u64r, l);
-    launch_early(k_pack2, gg, 256, 0, c->s, c->g, c->g64r, l.vh, l.npar);
+    launch_early(k_pack2, gg, 256, 0, c->s, c->g, c->g64r, l.vh, l.npar, odd_ns_of(l));
     c->launches += 3;
     // FP64 refinement
     unsigned reunit64 = o->refine_reunit ? o->refine_reunit : p->sweeps_to_reunitarization;

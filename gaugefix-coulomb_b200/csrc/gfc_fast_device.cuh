@@ -542,9 +542,18 @@ __device__ __forceinline__ void apply_backward(typename S::V *__restrict__ p, si
     }
 }
 
+// slot of the backward neighbour in direction d: checkerboard, or the odd-ns working
+// layout (odd_slot)
+template <bool CB>
+__device__ __forceinline__ uint32_t back_slot(const Lat &l, const Coord &c, int d) {
+    const uint32_t L = back_L(l, c, d);
+    if (CB) return L >> 1;
+    return odd_slot(l, L, d < 2 ? c.x : c.x ? c.x - 1 : (uint32_t)l.ns - 1);
+}
+
 // The e2 density of a site from its current links, without updating anything (the
-// "pre" of fast_site on its own).  CB = false: the lexicographic layout of odd ns
-// (one parity slot, i = the site's lexicographic index).
+// "pre" of fast_site on its own).  CB = false: odd ns (one parity slot; i = the site's
+// lexicographic index, its place in the fields odd_slot of it).
 template <class S, bool CB = true>
 __device__ __forceinline__ double measure_site(const typename S::V *__restrict__ u, const Lat &l, int par,
                                                uint32_t i) {
@@ -553,6 +562,7 @@ __device__ __forceinline__ double measure_site(const typename S::V *__restrict__
     if (!CB) par = 0;
     const int op = CB ? par ^ 1 : 0;
     Coord c = CB ? coord_cb(l, par, i) : coord_lex(l, i);
+    if (!CB) i = odd_slot(l, c.L, c.x);
     Mt<T> w;
 #pragma unroll
     for (int k = 0; k < 9; k++) w.e[k] = mkc<C>(T(0), T(0));
@@ -560,7 +570,7 @@ __device__ __forceinline__ double measure_site(const typename S::V *__restrict__
     for (int d = 0; d < 3; d++) {
         Mt<T> f, r;
         S::load(u + su_idx<S>(l, d, par, i), l.vh, f);
-        S::load(u + su_idx<S>(l, d, op, CB ? back_L(l, c, d) >> 1 : back_L(l, c, d)), l.vh, r);
+        S::load(u + su_idx<S>(l, d, op, back_slot<CB>(l, c, d)), l.vh, r);
 #pragma unroll
         for (int x = 0; x < 3; x++)
 #pragma unroll
@@ -774,8 +784,8 @@ __device__ __forceinline__ void apply_staged(const typename S::V *src, int sst, 
 // instead of from L2 (the links of the other directions are loaded from global
 // memory twice, as in fast_site).  Staged layout per CTA: entry e of matrix m of
 // thread x at sm[(m * NS + e) * BLOCK + x] (m = 2d forward, 2d+1 backward link of
-// direction d, m = NST for G).  Two-row storage only.  CB = false: the lexicographic
-// layout of odd ns (one parity slot, i = the site's lexicographic index).
+// direction d, m = NST for G).  Two-row storage only.  CB = false: odd ns (one parity
+// slot, i = the site's lexicographic index, its place in the fields odd_slot of it).
 // PROJ: the six links written are projected onto SU(3) first (apply_staged).
 template <class S, int BLOCK, bool SG, int NST = 6, bool CB = true, bool PROJ = false>
 __device__ __forceinline__ void fast_site_staged(typename S::V *__restrict__ u, typename S::V *__restrict__ g,
@@ -791,7 +801,8 @@ __device__ __forceinline__ void fast_site_staged(typename S::V *__restrict__ u, 
     Coord c = CB ? coord_cb(l, par, i) : coord_lex(l, i);
     uint32_t ib[3];
 #pragma unroll
-    for (int d = 0; d < 3; d++) ib[d] = CB ? back_L(l, c, d) >> 1 : back_L(l, c, d);
+    for (int d = 0; d < 3; d++) ib[d] = back_slot<CB>(l, c, d);
+    if (!CB) i = odd_slot(l, c.L, c.x);
     static_assert(NST == 2 || NST == 4 || NST == 6, "whole directions are staged");
     constexpr int ND = NST / 2;   // staged directions
     static_assert(!PROJ || ND == 3, "links are projected in the fully staged form only");

@@ -99,8 +99,9 @@ void launch_apply_gt(double2 *u, double2 *ut, const double2 *g, const Lat &l, in
 // format conversions over nblk SoA blocks of `stride` matrices (gfc_fast.cu)
 void launch_to_f32(const double2 *src, float4 *dst, uint32_t stride, uint32_t nblk, cudaStream_t s);
 void launch_identity32(float4 *g, uint32_t stride, uint32_t nblk, cudaStream_t s);
-void launch_pack2(const double2 *src, double2 *dst, uint32_t stride, uint32_t nblk, cudaStream_t s);
-void launch_unpack2(const double2 *src, double2 *dst, uint32_t stride, uint32_t nblk, cudaStream_t s);
+// (odd_ns: the lattice's ns if odd, 0 if even)
+void launch_pack2(const double2 *src, double2 *dst, uint32_t stride, uint32_t nblk, uint32_t odd_ns, cudaStream_t s);
+void launch_unpack2(const double2 *src, double2 *dst, uint32_t stride, uint32_t nblk, uint32_t odd_ns, cudaStream_t s);
 // seeded synthetic links built on the device (gfc_synth_dev.cu); gtmp is a
 // G-sized scratch field (overwritten)
 void launch_synth(const Lat &l, uint64_t seed, double scale, double2 *gtmp, double2 *u, double2 *ut,
