@@ -40,11 +40,11 @@ namespace gfc {
 enum : int { SS_EMPTY = 0, SS_FP32 = 1, SS_PEND = 2, SS_FP64 = 3, SS_DONE = 4, SS_VERIFY = 5, SS_LEX = 6 };
 // SS_LEX: a timeslice of an odd-ns lattice, FP64 on two stored rows in the odd-ns
 // working layout (odd_slot).  Same-parity sites meet across the periodic boundary there,
-// so a half-sweep runs as four launches over the boundary levels (the number of
-// coordinates equal to ns - 1), which keeps the order of the sequential z, y, x
-// sweep between every pair of sites that share a link; e2 is measured by a separate
-// pass over the state the half-sweep leaves (a site's post-update w is not final
-// when a later level updates a neighbour), so no verify pass is needed.
+// so a half-sweep takes them by boundary level (the number of coordinates equal to
+// ns - 1), which keeps the order of the sequential z, y, x sweep between every pair of
+// sites that share a link; e2 is measured by a separate pass over the state the
+// half-sweep leaves (a site's post-update w is not final when a later level updates a
+// neighbour), so no verify pass is needed.
 // SS_VERIFY: the FP64 e2 measured after half-sweep c - 1 fell below the tolerance, but
 // the timeslice has had half-sweep c too.  Its next pass measures e2 of the state it
 // is in without updating it: below the tolerance -> DONE with that state, else back
@@ -88,7 +88,7 @@ struct BState {
     int lex;              // 1: odd-ns slots may be active (their launches are in the round)
     int *counts;          // [0] n32 [1] n64 [2] npend [3] active timeslices [4] half-sweep k [5] overflow
                           // [6] [7] item cursors [8] [9] FP32 / FP64 reunitarisation due
-                          // [10] nlex [11..14] cursors of the odd-ns levels [15] of the odd-ns e2 pass
+                          // [10] nlex [11] cursor of the odd-ns sweep [15] of the odd-ns e2 pass
                           // [16] an FP32 rebuild due
     unsigned *status;
     double omega, switch_e2, tol;
@@ -389,17 +389,16 @@ __global__ void __launch_bounds__(32, MINB) k_bsweep_w(BState b) {
     }
 }
 
-// Odd-ns timeslices, boundary level `level` of one half-sweep: one-warp CTAs take
-// 32-site pieces of the level's sites of the half-sweep's parity (odd_level_site); the
-// items' further pieces have nothing to do.  Sites of one level share no link, and
-// every pair that does share one is in consecutive levels in the sequential sweep's
-// order (see SS_LEX).
+// Odd-ns timeslices, one half-sweep: one-warp CTAs take the pieces of a timeslice
+// (OddPieces; an item's BPIECES numbers that are past the last one have nothing to do)
+// and sweep each one's boundary levels in turn, which keeps the sequential sweep's
+// order between every pair of sites that share a link (see SS_LEX).
 template <int MINB>
-__global__ void __launch_bounds__(32, MINB) k_bsweep_lex(BState b, int level) {
+__global__ void __launch_bounds__(32, MINB) k_bsweep_lex(BState b) {
     grid_wait();
     extern __shared__ __align__(16) unsigned char bstage[];
     const int n = b.counts[10] * BPIECES;
-    int *cursor = b.counts + 11 + level;
+    int *cursor = b.counts + 11;
     const int lane = threadIdx.x;
     int it = 0;
     if (lane == 0) it = atomicAdd(cursor, 1);
@@ -409,21 +408,24 @@ __global__ void __launch_bounds__(32, MINB) k_bsweep_lex(BState b, int level) {
         if (lane == 0) ahead = atomicAdd(cursor, 1);
         const int2 item = b.itemslex[it / BPIECES];
         const int gid = item.x;
+        const int slot = gid / b.max_nt, t = gid - slot * b.max_nt;
+        const Lat l = b.slots[slot].l;
+        uint32_t k = (uint32_t)(item.y * BPIECES + it % BPIECES);
         // ns = 1: every spatial link closes on its own site and e2 vanishes identically,
         // so the fix leaves the lattice as it is (the half-sweeps pass it by until its
         // first e2 measurement retires it)
-        const int slot = gid / b.max_nt, t = gid - slot * b.max_nt;
-        const BSlot &sl = b.slots[slot];
-        const uint32_t k = (uint32_t)item.y * BCHUNK + (uint32_t)(it % BPIECES) * 32 + lane;
-        const uint32_t count = odd_level_count(sl.l, level);
-        if (k - lane < count && *(volatile int *)&b.state[gid] == SS_LEX && sl.l.ns > 1) {   // uniform in the CTA
+        if (l.ns > 1 && k < OddPieces(l).count() && *(volatile int *)&b.state[gid] == SS_LEX) {   // uniform
             const int par = b.sweeps[gid] & 1;
-            const Lat l = sl.l;
-            uint32_t off;
-            if (k < count && odd_level_site(l, par, (uint32_t)t, level, k, off)) {
-                double a = 0.0, z = 0.0;
-                fast_site_staged<S64R, 32, false, 6, false>(sl.u64r, sl.g64r, l, 0, (uint32_t)t * l.vs + off, b.omega,
-                                                             b.hits, 0, a, z, (double2 *)bstage);
+            const int kind = OddPieces(l).kind(k);
+            double2 *u = b.slots[slot].u64r, *g = b.slots[slot].g64r;
+#pragma unroll 1
+            for (int level = 0; level <= 3 - kind; level++) {
+                uint32_t off;
+                double pre = 0.0, post = 0.0;
+                if (odd_piece_site(l, par, (uint32_t)t, kind, k, lane, level, off))
+                    fast_site_staged<S64R, 32, false, 6, false>(u, g, l, 0, (uint32_t)t * l.vs + off, b.omega, b.hits,
+                                                                 0, pre, post, (double2 *)bstage);
+                if (level < 3 - kind) odd_level_fence();
             }
         }
         it = __shfl_sync(0xffffffffu, ahead, 0);
@@ -431,7 +433,7 @@ __global__ void __launch_bounds__(32, MINB) k_bsweep_lex(BState b, int level) {
 }
 
 // e2 of the odd-ns timeslices measured on this half-sweep (mflag MF_NOW), over all
-// their sites, on the state the four level launches left: one partial per piece.
+// their sites, on the state the sweep left: one partial per piece.
 __global__ void __launch_bounds__(32) k_bmeasure_lex(BState b) {
     grid_wait();
     const int n = b.counts[10];
@@ -612,11 +614,13 @@ __device__ __forceinline__ void breunit_part(const BState &b, unsigned period, i
     const int2 *items = lex ? b.itemslex : (F64 ? b.items64 : b.items32);
     const int expect = lex ? SS_LEX : (F64 ? SS_FP64 : SS_FP32);
     // the CTA examines BCHUNK items at once (one per thread) and projects only the
-    // chunks of timeslices that are due; most half-sweeps none are
-    for (int base = blockIdx.x * BCHUNK; base < n; base += gridDim.x * BCHUNK) {
+    // chunks of timeslices that are due; most half-sweeps none are.  CTA c takes items c,
+    // c + gridDim.x, ...: all of a small batch is often due at once, and items handed out
+    // BCHUNK in a row left it to a few CTAs (12 small lattices: 817 us, now 37).
+    for (int base = blockIdx.x; base < n; base += gridDim.x * BCHUNK) {
         if (threadIdx.x == 0) ndue = 0;
         __syncthreads();
-        const int it = base + threadIdx.x;
+        const int it = base + (int)threadIdx.x * (int)gridDim.x;
         if (it < n) {
             const int gid = items[it].x;
             const int own = b.sweeps[gid];
@@ -672,10 +676,10 @@ __global__ void __launch_bounds__(BCHUNK) k_brefresh(BState b) {
     __shared__ int ndue;
     if (!b.refresh32 || !b.counts[16]) return;   // uniform
     const int n = b.counts[0];
-    for (int base = blockIdx.x * BCHUNK; base < n; base += gridDim.x * BCHUNK) {
+    for (int base = blockIdx.x; base < n; base += gridDim.x * BCHUNK) {   // spread as in breunit_part
         if (threadIdx.x == 0) ndue = 0;
         __syncthreads();
-        const int it = base + threadIdx.x;
+        const int it = base + (int)threadIdx.x * (int)gridDim.x;
         if (it < n) {
             const int gid = b.items32[it].x;
             const int own = b.sweeps[gid];
@@ -1236,12 +1240,12 @@ static void launch_bsweep_k(int grid, cudaStream_t st, const BState &bs) {
     launch_early(kern, grid, BCHUNK, bytes, st, bs);
 }
 
-static void launch_bsweep_lex(int grid, cudaStream_t st, const BState &bs, int level) {
+static void launch_bsweep_lex(int grid, cudaStream_t st, const BState &bs) {
     constexpr size_t bytes = (size_t)6 * S64R::NS * 32 * 16;
     auto kern = k_bsweep_lex<11>;
     static std::atomic<unsigned long long> done{0};
     smem_attr_once(done, kern, bytes);
-    launch_early(kern, grid, 32, bytes, st, bs, level);
+    launch_early(kern, grid, 32, bytes, st, bs);
 }
 
 template <int MINB>
@@ -1318,8 +1322,8 @@ static void enqueue_round(gfc_batch *b, const BState &bs) {
             launch_bsweep<S64R>(m64, b->stage64 != 0, b->nsm * m64, st, bs);
         }
         if (bs.lex) {
-            // odd-ns timeslices: the four boundary levels in order, then their e2
-            for (int level = 0; level < 4; level++) launch_bsweep_lex(b->nsm * 11, st, bs, level);
+            // odd-ns timeslices, then their e2
+            launch_bsweep_lex(b->nsm * 11, st, bs);
             launch_early(k_bmeasure_lex, b->nsm * 16, 32, 0, st, bs);
         }
         launch_early(k_bslice, (b->nslices + 7) / 8, 256, 0, st, bs);
@@ -1364,7 +1368,7 @@ extern "C" int gfc_batch_round(gfc_batch *b, const gfc_params *p, const gfc_opti
     int rc = ensure_graph(b, p, o);
     if (rc) return rc;
     GFC_CHECK(cudaGraphLaunch(b->exec, b->s));
-    b->launches += 4 + ((b->minb32 > 4 && b->minb64 > 4 ? 3 : 4) + (b->odd_slots > 0 ? 5 : 0) +
+    b->launches += 4 + ((b->minb32 > 4 && b->minb64 > 4 ? 3 : 4) + (b->odd_slots > 0 ? 2 : 0) +
                         (o->fp32_refresh > 0 ? 2 : 0)) * b->round_k;
     b->rounds++;
     GFC_CHECK(cudaMemcpyAsync(b->hcounts, b->counts, sizeof(int) * 8, cudaMemcpyDeviceToHost, b->s));

@@ -158,6 +158,82 @@ __host__ __device__ __forceinline__ bool odd_level_site(const Lat &l, int p, uin
     return true;
 }
 
+// The same half-sweep as one launch.  The sites fall into components, those that agree up
+// to 0 <-> e in some coordinates, which share no link with one another; with D
+// coordinates 0 or e a component has 2^D sites, to be updated by level:
+//   kind 0, corner (D = 3): levels of 1, 3, 3, 1 sites, one component per timeslice (of
+//           its parity);
+//   kind 1, edges (D = 2): levels of 1, 2, 1 sites;
+//   kind 2, faces (D = 1): levels of 1 and 1 sites;
+//   kind 3, inner (D = 0): one site.
+// One warp takes a piece of a timeslice, up to 1, 16, 32 or 32 components of a kind, and
+// sweeps its levels in turn, ordered by its own fences.  This saves three launches, each
+// as long as a warp's chain of instructions, but its inner and face pieces split the
+// rows of level 0 (x = 0 leaves them), which costs a lattice that streams from HBM more
+// than it gains: see the rules at its launches.  (The free coordinates run over [1, e),
+// an odd number of values, so the sites of a parity are numbered by pairs of rows, as
+// such rows alternate.)
+struct OddPieces {
+    uint32_t edge, face, inner;      // pieces of a timeslice by kind (corner: 1)
+    __host__ __device__ explicit OddPieces(const Lat &l) {
+        const uint32_t m = (uint32_t)l.ns - 2;   // ns >= 3
+        edge = (3 * ((m + 1) / 2) + 15) / 16;
+        face = (3 * ((m * m + 1) / 2) + 31) / 32;
+        inner = ((m * m * m + 1) / 2 + 31) / 32;
+    }
+    __host__ __device__ uint32_t count() const { return 1 + edge + face + inner; }
+    // kind of piece k < count(), k becoming its number within the kind
+    __host__ __device__ int kind(uint32_t &k) const {
+        if (k < 1) return 0;
+        if ((k -= 1) < edge) return 1;
+        if ((k -= edge) < face) return 2;
+        k -= face;
+        return 3;
+    }
+};
+// The site (its index inside the timeslice) that `lane` updates on `level` of piece k of a
+// kind, parity p, timeslice t; false where it has none.  Levels 0 .. 3 - kind.
+__host__ __device__ __forceinline__ bool odd_piece_site(const Lat &l, int p, uint32_t t, int kind, uint32_t k,
+                                                        uint32_t lane, int level, uint32_t &off) {
+    const uint32_t ns = (uint32_t)l.ns, e = ns - 1, m = ns - 2, q = ((uint32_t)p ^ t) & 1u;
+    uint32_t c[3] = {0, 0, 0};   // x, y, z
+    if (kind == 3) {
+        const uint32_t j = k * 32 + lane, q1 = q ^ 1u, a = q1 ? (m - 1) >> 1 : (m + 1) >> 1;
+        const uint32_t pair = j / m, rem = j - pair * m, R = rem < a ? 2 * pair : 2 * pair + 1;
+        const uint32_t z = R / m, y = R - z * m;
+        if (z >= m) return false;
+        c[0] = 1 + 2 * (rem < a ? rem : rem - a) + (q1 ^ (R & 1u));
+        c[1] = 1 + y;
+        c[2] = 1 + z;
+    } else if (kind == 2) {
+        const uint32_t n = (m * m + 1) / 2, i = k * 32 + lane, f = i / n, j = i - f * n;
+        const uint32_t a = q ? (m - 1) >> 1 : (m + 1) >> 1;
+        const uint32_t pair = j / m, rem = j - pair * m, R = rem < a ? 2 * pair : 2 * pair + 1;
+        if (f > 2 || R >= m) return false;
+        c[f] = level ? e : 0;
+        c[f == 0 ? 1 : 0] = 1 + 2 * (rem < a ? rem : rem - a) + (q ^ (R & 1u));
+        c[f == 2 ? 1 : 2] = 1 + R;
+    } else if (kind == 1) {
+        const uint32_t n = (m + 1) / 2, i = k * 16 + (lane >> 1), f = i / n, v = 2 * (i - f * n) + (q ^ 1u);
+        if (f > 2 || v >= m || (level != 1 && (lane & 1u))) return false;
+        c[f] = 1 + v;
+        if (level == 2 || (level == 1 && !(lane & 1u))) c[f == 0 ? 1 : 0] = e;
+        if (level == 2 || (level == 1 && (lane & 1u))) c[f == 2 ? 1 : 2] = e;
+    } else {
+        if (q || lane >= (level == 0 || level == 3 ? 1u : 3u)) return false;
+        for (uint32_t d = 0; d < 3; d++)
+            if (level == 3 || (level == 1 && lane == d) || (level == 2 && lane != d)) c[d] = e;
+    }
+    off = (c[2] * ns + c[1]) * ns + c[0];
+    return true;
+}
+// Between two levels of a piece: what the warp's lanes have stored, every lane reads
+// (through L2 too, where cp.async fetches links).
+__device__ __forceinline__ void odd_level_fence() {
+    __threadfence();
+    __syncwarp();
+}
+
 __host__ __device__ __forceinline__ uint32_t fwd_L(const Lat &l, const Coord &c, int d) {
     uint32_t ns = l.ns;
     if (d == 0) return c.z + 1 < ns ? c.L + ns * ns : c.L - (ns - 1) * ns * ns;

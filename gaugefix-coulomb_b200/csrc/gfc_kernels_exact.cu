@@ -215,6 +215,28 @@ __global__ void __launch_bounds__(LEVEL_BLOCK, 8) k_sweep_exact_level(double2 *_
         site_update_exact_staged<LEVEL_BLOCK, false>(u, g, l, 0, c, omega, hits, (double2 *)level_stage);
 }
 
+// The same half-sweep in one launch, a warp to a piece (OddPieces): 15^3 x 32 53 us per
+// half-sweep where the four launches take 79, 31^3 x 64 773 us where they take 660.
+__global__ void __launch_bounds__(LEVEL_BLOCK, 8) k_sweep_exact_pieces(double2 *__restrict__ u,
+                                                                      double2 *__restrict__ g, Lat l, int sweep,
+                                                                      double omega, unsigned hits,
+                                                                      const unsigned *stop) {
+    extern __shared__ __align__(16) unsigned char level_stage[];
+    grid_wait();
+    if (stop && *(volatile const unsigned *)stop) return;
+    uint32_t k = blockIdx.x / l.nt;   // the longest pieces (corners, edges) first
+    const uint32_t t = blockIdx.x - k * l.nt;
+    const int kind = OddPieces(l).kind(k);
+#pragma unroll 1
+    for (int level = 0; level <= 3 - kind; level++) {
+        uint32_t off;
+        if (odd_piece_site(l, sweep & 1, t, kind, k, threadIdx.x, level, off))
+            site_update_exact_staged<LEVEL_BLOCK, false>(u, g, l, 0, coord_lex(l, t * l.vs + off), omega, hits,
+                                                         (double2 *)level_stage);
+        if (level < 3 - kind) odd_level_fence();
+    }
+}
+
 int exact_num_shapes() { return 5; }
 
 // returns the number of kernels launched
@@ -244,6 +266,15 @@ int launch_sweep_exact(double2 *u, double2 *g, const Lat &l, int sweep, double o
         constexpr size_t bytes = (size_t)6 * 9 * LEVEL_BLOCK * sizeof(double2);
         static std::atomic<unsigned long long> done{0};
         smem_attr_once(done, k_sweep_exact_level, bytes);
+        // one launch up to two waves of its warps (8 per SM), where a launch is a warp's
+        // chain of instructions; level by level where the sectors of whole rows count
+        if (l.ns > 1 && OddPieces(l).count() * (uint32_t)l.nt <= 2 * 8 * 148) {
+            static std::atomic<unsigned long long> done_p{0};
+            smem_attr_once(done_p, k_sweep_exact_pieces, bytes);
+            launch_early(k_sweep_exact_pieces, OddPieces(l).count() * l.nt, LEVEL_BLOCK, bytes, s, u, g, l, sweep,
+                         omega, hits, stop);
+            return 1;
+        }
         int launched = 0;
         for (int level = l.ns == 1 ? 3 : 0; level < 4; level++, launched++)   // ns = 1: corners only
             launch_early(k_sweep_exact_level, (odd_level_count(l, level) * l.nt + LEVEL_BLOCK - 1) / LEVEL_BLOCK,

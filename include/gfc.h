@@ -274,7 +274,7 @@ int  gfc_e2_theta_device_noalloc(int ns, int nt, const double *u_dev, void *stre
  * tolerance (measured on the links it keeps); with GFC_PREC_MIXED it first runs FP32
  * bulk sweeps until its e2 falls below options.switch_e2 and is then rebuilt in
  * FP64.  Lattices of odd ns run in FP64 whatever the precision asked for, each
- * half-sweep in four launches over the boundary levels that keep the reference's
+ * half-sweep in two launches over the boundary levels that keep the reference's
  * sequential order where same-parity sites share a link.  One round = K
  * half-sweeps of all active timeslices, replayed as a captured CUDA graph.  Slots
  * can be added, activated, finalised and removed between rounds (continuous
