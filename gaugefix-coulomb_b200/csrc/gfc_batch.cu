@@ -834,6 +834,8 @@ using namespace gfc;
 struct gfc_batch {
     int dev = 0;
     cudaStream_t s = nullptr;
+    cudaStream_t s2 = nullptr;       // the odd-ns branch of a captured round
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     int max_slots = 0, max_nt = 0, nslices = 0;
     size_t max_sites = 0, used_sites = 0;
     std::vector<BSlot> hs;          // host copies of the descriptors
@@ -897,6 +899,9 @@ extern "C" int gfc_batch_create(int device, size_t max_sites, int max_slots, int
     }
     BTRY(cudaSetDevice(device));
     BTRY(cudaStreamCreateWithFlags(&b->s, cudaStreamNonBlocking));
+    BTRY(cudaStreamCreateWithFlags(&b->s2, cudaStreamNonBlocking));
+    BTRY(cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming));
+    BTRY(cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming));
     BTRY(cudaMalloc(&b->dslots, sizeof(BSlot) * max_slots));
     BTRY(cudaMemset(b->dslots, 0, sizeof(BSlot) * max_slots));
     BTRY(cudaMalloc(&b->state, sizeof(int) * b->nslices));
@@ -978,6 +983,9 @@ extern "C" int gfc_batch_destroy(gfc_batch *b) {
     cudaFreeHost(b->hstate);
     cudaFreeHost(b->hres);
     if (b->s) cudaStreamDestroy(b->s);
+    if (b->s2) cudaStreamDestroy(b->s2);
+    if (b->ev_fork) cudaEventDestroy(b->ev_fork);
+    if (b->ev_join) cudaEventDestroy(b->ev_join);
     delete b;
     return GFC_OK;
 }
@@ -1304,13 +1312,24 @@ static void launch_bsweep(int minb, bool stage, int grid, cudaStream_t st, const
 }
 
 // enqueue one round on the stream (used for capture)
-static void enqueue_round(gfc_batch *b, const BState &bs) {
+static cudaError_t enqueue_round(gfc_batch *b, const BState &bs) {
     cudaStream_t st = b->s;
+    cudaError_t e;
     launch_early(k_compact, 1, 1024, 0, st, bs);
     launch_early(k_switch_g, b->grid, BCHUNK, 0, st, bs);
     launch_early(k_switch_u, b->grid, BCHUNK, 0, st, bs);
     launch_early(k_switch_done, (b->nslices + 255) / 256, 256, 0, st, bs);
     for (int k = 0; k < b->round_k; k++) {
+        if (bs.lex) {
+            // odd-ns timeslices, then their e2, on a branch beside the other sweeps (other
+            // timeslices, other counters); first, so that its long chains start at once
+            if ((e = cudaEventRecord(b->ev_fork, st)) != cudaSuccess ||
+                (e = cudaStreamWaitEvent(b->s2, b->ev_fork, 0)) != cudaSuccess)
+                return e;
+            launch_bsweep_lex(b->nsm * 11, b->s2, bs);
+            launch_early(k_bmeasure_lex, b->nsm * 16, 32, 0, b->s2, bs);
+            if ((e = cudaEventRecord(b->ev_join, b->s2)) != cudaSuccess) return e;
+        }
         // one resident wave of persistent CTAs: a CTA that had to wait for a slot
         // would start its share of the items late and stretch the tail
         if (b->minb32 > 4 && b->minb64 > 4) {
@@ -1321,11 +1340,7 @@ static void enqueue_round(gfc_batch *b, const BState &bs) {
             launch_bsweep<S32>(b->minb32, false, b->nsm * b->minb32, st, bs);
             launch_bsweep<S64R>(m64, b->stage64 != 0, b->nsm * m64, st, bs);
         }
-        if (bs.lex) {
-            // odd-ns timeslices, then their e2
-            launch_bsweep_lex(b->nsm * 11, st, bs);
-            launch_early(k_bmeasure_lex, b->nsm * 16, 32, 0, st, bs);
-        }
+        if (bs.lex && (e = cudaStreamWaitEvent(st, b->ev_join, 0)) != cudaSuccess) return e;
         launch_early(k_bslice, (b->nslices + 7) / 8, 256, 0, st, bs);
         launch_early(k_breunit, b->grid, BCHUNK, 0, st, bs);
         if (bs.refresh32) {
@@ -1333,6 +1348,7 @@ static void enqueue_round(gfc_batch *b, const BState &bs) {
             launch_early(k_brefresh<1>, b->grid, BCHUNK, 0, st, bs);
         }
     }
+    return cudaSuccess;
 }
 
 static int ensure_graph(gfc_batch *b, const gfc_params *p, const gfc_options *o) {
@@ -1347,8 +1363,9 @@ static int ensure_graph(gfc_batch *b, const gfc_params *p, const gfc_options *o)
         b->graph = nullptr;
     }
     GFC_CHECK(cudaStreamBeginCapture(b->s, cudaStreamCaptureModeThreadLocal));
-    enqueue_round(b, bs);
+    const cudaError_t e = enqueue_round(b, bs);
     GFC_CHECK(cudaStreamEndCapture(b->s, &b->graph));
+    GFC_CHECK(e);
     GFC_CHECK(cudaGraphInstantiate(&b->exec, b->graph, 0));
     b->captured = bs;
     return GFC_OK;
