@@ -119,8 +119,8 @@ extern "C" int gfc_ctx_create(int ns, int nt, int device, int flags, gfc_ctx **o
         c->part_n = (size_t)nt * nbx * 4;
         TRY(cudaMalloc(&c->part, c->part_n * sizeof(double)));
         TRY(cudaMalloc(&c->dres, 32 * sizeof(double)));
-        TRY(cudaMalloc(&c->dstatus, sizeof(unsigned)));
-        TRY(cudaMemset(c->dstatus, 0, sizeof(unsigned)));
+        TRY(cudaMalloc(&c->dstatus, 2 * sizeof(unsigned)));
+        TRY(cudaMemset(c->dstatus, 0, 2 * sizeof(unsigned)));
         TRY(cudaMalloc(&c->e2_slice, (size_t)nt * 2 * sizeof(double)));
         TRY(cudaMallocHost(&c->hres, 32 * sizeof(double)));
         TRY(cudaEventCreate(&c->ev_a));
@@ -434,8 +434,8 @@ static int read_results(gfc_ctx *c, int n) {
 // e2 (calculate_e2) and theta (calculateTheta) of the current spatial links.
 static int obs_e2_theta(gfc_ctx *c, double *e2, double *theta, double *slices) {
     const Lat &l = c->lat;
-    launch_obs(c->u, l, c->part, c->dres, c->e2_slice, c->s);
-    c->launches += 2;
+    launch_obs(c->u, l, c->part, c->dstatus + 1, c->dres, c->e2_slice, c->s);
+    c->launches++;
     GFC_CHECK(cudaGetLastError());
     int rc = read_results(c, 2);
     if (rc) return rc;
@@ -475,8 +475,8 @@ extern "C" int gfc_ctx_functional(gfc_ctx *c, double *F) {
     if (!c->has_links) return GFC_ERR_STATE;
     GFC_CHECK(cudaSetDevice(c->dev));
     const Lat &l = c->lat;
-    launch_functional(c->u, l, c->part, c->dres, c->s);
-    c->launches += 2;
+    launch_functional(c->u, l, c->part, c->dstatus + 1, c->dres, c->s);
+    c->launches++;
     GFC_CHECK(cudaGetLastError());
     int rc = read_results(c, 1);
     if (rc) return rc;
@@ -489,8 +489,8 @@ extern "C" int gfc_ctx_plaquette(gfc_ctx *c, double *spatial, double *temporal) 
     if (!c->has_links) return GFC_ERR_STATE;
     GFC_CHECK(cudaSetDevice(c->dev));
     const Lat &l = c->lat;
-    launch_plaquette(c->u, c->ut, l, c->part, c->dres, c->s);
-    c->launches += 2;
+    launch_plaquette(c->u, c->ut, l, c->part, c->dstatus + 1, c->dres, c->s);
+    c->launches++;
     GFC_CHECK(cudaGetLastError());
     int rc = read_results(c, 2);
     if (rc) return rc;
@@ -627,7 +627,7 @@ static int fix_reference_schedule(gfc_ctx *c, const gfc_params *p, const gfc_opt
 // Exact kernel with the proxy evaluated after every half-sweep (standalone
 // reduction, one host wait per half-sweep): reference arithmetic, earliest stop.
 // Reference arithmetic, the proxy measured exactly (as calculate_e2 / calculateTheta
-// do), near the tolerance after every half-sweep.  The test runs on the device: a check kernel after each
+// do), near the tolerance after every half-sweep.  The test runs on the device: the last block of a
 // half-sweep's observables sets a stop word, after which the queued sweep and
 // observables launches do nothing, so the links returned are those whose proxy was
 // found below the tolerance.  The host reads the stop word every 32 half-sweeps and
@@ -666,9 +666,9 @@ static int fix_every_sweep_exact(gfc_ctx *c, const gfc_params *p, const gfc_opti
         for (; sweep < end; sweep++) {
             c->launches += launch_sweep_exact(c->u, c->g, l, sweep, omega, p->hits, c->s, c->shape_exact, stop);
             if (dense || sweep + 1 == end) {
-                launch_obs(c->u, l, c->part, c->dres, nullptr, c->s, stop);
-                launch_exact_check(c->dres, l, theta, p->tolerance, sweep + 1, stop, c->s);
-                c->launches += 3;
+                launch_obs(c->u, l, c->part, c->dstatus + 1, c->dres, nullptr, c->s, stop, theta, p->tolerance,
+                           sweep + 1);
+                c->launches++;
             }
         }
         GFC_CHECK(cudaMemcpyAsync(c->hres + 16, stop, sizeof(unsigned), cudaMemcpyDeviceToHost, c->s));

@@ -923,8 +923,8 @@ extern "C" int gfc_batch_create(int device, size_t max_sites, int max_slots, int
     BTRY(cudaMalloc(&b->itemslex, sizeof(int2) * b->cap_pend));   // chunks over whole timeslices
     BTRY(cudaMalloc(&b->counts, sizeof(int) * 17));
     BTRY(cudaMemset(b->counts, 0, sizeof(int) * 17));
-    BTRY(cudaMalloc(&b->status, sizeof(unsigned)));
-    BTRY(cudaMemset(b->status, 0, sizeof(unsigned)));
+    BTRY(cudaMalloc(&b->status, 2 * sizeof(unsigned)));   // [1]: ticket of the observables
+    BTRY(cudaMemset(b->status, 0, 2 * sizeof(unsigned)));
     BTRY(cudaMallocHost(&b->hcounts, sizeof(int) * 8));
     BTRY(cudaMallocHost(&b->hstate, sizeof(int) * b->nslices));
     BTRY(cudaMalloc(&b->dres, sizeof(double) * 8));
@@ -1435,9 +1435,9 @@ extern "C" int gfc_batch_finalize(gfc_batch *b, int slot, gfc_report *r) {
         std::vector<int> sw(l.nt);
         GFC_CHECK(cudaMemcpyAsync(sw.data(), b->sweeps + (size_t)slot * b->max_nt, sizeof(int) * l.nt,
                                   cudaMemcpyDeviceToHost, b->s));
-        launch_obs(sl.u, l, b->part, b->dres, nullptr, b->s);
-        launch_functional(sl.u, l, b->part, b->dres + 2, b->s);
-        b->launches += 4;
+        launch_obs(sl.u, l, b->part, b->status + 1, b->dres, nullptr, b->s);
+        launch_functional(sl.u, l, b->part, b->status + 1, b->dres + 2, b->s);
+        b->launches += 2;
         GFC_CHECK(cudaMemcpyAsync(b->hres, b->dres, sizeof(double) * 3, cudaMemcpyDeviceToHost, b->s));
         GFC_CHECK(cudaStreamSynchronize(b->s));
         int mx = 0;
@@ -1466,7 +1466,7 @@ extern "C" int gfc_batch_plaquette(gfc_batch *b, int slot, double *spatial, doub
     if (rc) return rc;
     GFC_CHECK(cudaSetDevice(b->dev));
     const BSlot &sl = b->hs[slot];
-    launch_plaquette(sl.u, sl.ut, sl.l, b->part, b->dres, b->s);
+    launch_plaquette(sl.u, sl.ut, sl.l, b->part, b->status + 1, b->dres, b->s);
     GFC_CHECK(cudaMemcpyAsync(b->hres, b->dres, sizeof(double) * 2, cudaMemcpyDeviceToHost, b->s));
     GFC_CHECK(cudaStreamSynchronize(b->s));
     if (spatial) *spatial = b->hres[0] / (3.0 * (double)sl.l.v);

@@ -27,7 +27,7 @@ struct gfc_ctx {
     size_t part_n = 0;
     double *dres = nullptr;       // [32] device results
     double *hres = nullptr;       // [32] pinned mirror
-    unsigned *dstatus = nullptr;
+    unsigned *dstatus = nullptr;  // [0] status word, [1] ticket of the observables (zero between launches)
     double *e2_slice = nullptr;   // [nt] per-timeslice e2 partials (fused path)
     double *e2_hist = nullptr;    // [2][hist_n] per half-sweep fused e2 (two parity halves)
     int hist_n = 0;

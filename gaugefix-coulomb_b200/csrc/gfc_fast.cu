@@ -36,6 +36,7 @@
 #include "gfc_fast.h"
 
 #include "gfc_fast_device.cuh"
+#include "gfc_reduce.cuh"
 
 namespace gfc {
 
@@ -683,12 +684,14 @@ static void launch_halfsweep_lex_fast(gfc_ctx *c, int sweep, double omega, unsig
 
 // e2 and theta partials (theta = e2 / 6 identically) per timeslice of the two-row links of
 // odd ns, in the order of their slots: grid (nbx, nt), fixed summation order
+// (the stop test of k_obs)
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_e2_lex_fast(const double2 *__restrict__ u, Lat l,
-                                                       double *__restrict__ part, const unsigned *stop) {
+                                                       double *__restrict__ part, unsigned *__restrict__ ticket,
+                                                       double *__restrict__ out, unsigned *stop, int theta,
+                                                       double tol, int sweep) {
     grid_wait();
     if (stop && *(volatile const unsigned *)stop) return;
-    __shared__ double sh[2][BLOCK / 32];
     const uint32_t t = blockIdx.y;
     double v[2] = {0.0, 0.0};
     for (uint32_t k = blockIdx.x * BLOCK + threadIdx.x; k < l.vs; k += gridDim.x * BLOCK) {
@@ -696,20 +699,20 @@ __global__ void __launch_bounds__(BLOCK) k_e2_lex_fast(const double2 *__restrict
         v[0] += e2;
         v[1] += 0.5 * e2;   // Re Tr(div A div A^dagger) of the site
     }
-    fblock_sum<BLOCK, 2>(v, sh);
-    if (threadIdx.x == 0) {
-        const size_t o = ((size_t)t * gridDim.x + blockIdx.x) * 2;
-        part[o] = v[0];
-        part[o + 1] = v[1];
+    block_sum<2>(v);
+    if (last_block_sum<2>(v, part, ticket, nullptr)) {
+        out[0] = v[0];
+        out[1] = v[1];
+        const double n = (double)l.v, res = theta ? v[1] / (3.0 * n) : v[0] / n;
+        if (stop && res <= tol) *stop = (unsigned)sweep;
     }
 }
 
-static void launch_e2_lex_fast(gfc_ctx *c, const unsigned *stop) {
+static void launch_e2_lex_fast(gfc_ctx *c, unsigned *stop, int theta, double tol, int sweep) {
     const Lat &l = c->lat;
-    const int nbx = obs_blocks_per_slice(l);
-    launch_early(k_e2_lex_fast<128>, dim3(nbx, l.nt), 128, 0, c->s, c->u64r, l, c->part, stop);
-    launch_finalize2(c->part, l, nbx, c->dres, c->s, stop);
-    c->launches += 2;
+    launch_early(k_e2_lex_fast<128>, dim3(obs_blocks_per_slice(l), l.nt), 128, 0, c->s, c->u64r, l, c->part,
+                 c->dstatus + 1, c->dres, stop, theta, tol, sweep);
+    c->launches++;
 }
 
 // n half-sweeps from `first` on the two stored rows (packed before, unpacked after),
@@ -758,9 +761,7 @@ int fix_every_sweep_odd_fast(gfc_ctx *c, const gfc_params *p, const gfc_options 
         for (; sweep < end; sweep++) {
             launch_halfsweep_lex_fast(c, sweep, omega, p->hits, stop);
             if (dense || sweep + 1 == end) {
-                launch_e2_lex_fast(c, stop);
-                launch_exact_check(c->dres, l, theta, p->tolerance, sweep + 1, stop, c->s);
-                c->launches++;
+                launch_e2_lex_fast(c, stop, theta, p->tolerance, sweep + 1);
             }
         }
         GFC_CHECK(cudaMemcpyAsync(c->hres + 16, stop, sizeof(unsigned), cudaMemcpyDeviceToHost, c->s));

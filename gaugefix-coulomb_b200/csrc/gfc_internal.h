@@ -67,13 +67,11 @@ int exact_num_shapes();
 void launch_reunitarize(double2 *base, uint32_t stride, uint32_t nblk, unsigned *status, cudaStream_t s);
 void launch_identity(double2 *g, const Lat &l, cudaStream_t s);
 int obs_blocks_per_slice(const Lat &l);
-void launch_finalize2(const double *part, const Lat &l, int nbx, double *out, cudaStream_t s, const unsigned *stop);
-void launch_obs(const double2 *u, const Lat &l, double *part, double *out, double *slice_out, cudaStream_t s,
-                const unsigned *stop = nullptr);
-// proxy of out (launch_obs) <= tol sets *stop = sweep (once)
-void launch_exact_check(const double *out, const Lat &l, int theta, double tol, int sweep, unsigned *stop,
-                        cudaStream_t s);
-void launch_functional(const double2 *u, const Lat &l, double *part, double *out, cudaStream_t s);
+// sums of e2 and theta densities into out[0..1] (and per timeslice); part: scratch of
+// 2 nt obs_blocks_per_slice doubles, ticket: a zero word.  stop, theta, tol, sweep: k_obs
+void launch_obs(const double2 *u, const Lat &l, double *part, unsigned *ticket, double *out, double *slice_out,
+                cudaStream_t s, unsigned *stop = nullptr, int theta = 0, double tol = 0.0, int sweep = 0);
+void launch_functional(const double2 *u, const Lat &l, double *part, unsigned *ticket, double *out, cudaStream_t s);
 
 // ---- layout transforms (gfc_kernels_io.cu)
 // Raw file bytes (reference AoS order, elem_bytes 8 or 4, optionally big endian)
@@ -107,7 +105,7 @@ void launch_unpack2(const double2 *src, double2 *dst, uint32_t stride, uint32_t 
 void launch_synth(const Lat &l, uint64_t seed, double scale, double2 *gtmp, double2 *u, double2 *ut,
                   cudaStream_t s);
 // plaquette partials: [nt][nbx][2] = (spatial sum, temporal sum) of Re Tr/3
-void launch_plaquette(const double2 *u, const double2 *ut, const Lat &l, double *part, double *out,
+void launch_plaquette(const double2 *u, const double2 *ut, const Lat &l, double *part, unsigned *ticket, double *out,
                       cudaStream_t s);
 
 // ---- batch internals shared with the request server (gfc_batch.cu)

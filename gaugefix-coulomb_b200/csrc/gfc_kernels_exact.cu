@@ -12,10 +12,13 @@
 // their transformation is applied once at the end (k_temporal_transform).
 //
 // Memory traffic per site-update: 6 links + G read and written = 14 x 144 B.
+#include <algorithm>
+
 #include "gfc_device.cuh"
 #include "gfc.h"
 #include "gfc_ctx.h"
 #include "gfc_internal.h"
+#include "gfc_reduce.cuh"
 
 namespace gfc {
 
@@ -321,102 +324,26 @@ void launch_identity(double2 *g, const Lat &l, cudaStream_t s) {
 }
 
 // ------------------------------------------------------------- observables --
-// Per site: div A (four_potential.c:70-113) -> e2 density sum_a c_a^2
-// (gauge_fixing.c:428-438) and theta density Re Tr(divA divA^dag)
-// (gauge_fixing.c:374-380); block partials per timeslice.
-__device__ __forceinline__ void calc_A(const M3 &u, M3 &A) {
-    // subtractionHermConjTrless3x3 (SU3_ops.c:322-372) then * (-i/2)
-    M3 d;
-    double2 tr = cz();
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        d.e[EL(a, a)] = make_double2(0.0, xm(2.0, u.e[EL(a, a)].y));
-        tr = xcadd(tr, d.e[EL(a, a)]);
-    }
-    tr = make_double2(xd(tr.x, 3.0), xd(tr.y, 3.0));
-#pragma unroll
-    for (int a = 0; a < 3; a++) d.e[EL(a, a)] = xcsub(d.e[EL(a, a)], tr);
-#pragma unroll
-    for (int a = 0; a < 3; a++)
-#pragma unroll
-        for (int b = 0; b < 3; b++)
-            if (a != b) d.e[EL(a, b)] = xcsub(u.e[EL(a, b)], cconj(u.e[EL(b, a)]));
-    const double2 al = make_double2(-0.0, -0.5);
-#pragma unroll
-    for (int k = 0; k < 9; k++) A.e[k] = xcmul(al, d.e[k]);
-}
-
+// Per site: div A (four_potential.c:70-113) -> e2 and theta densities (gfc_reduce.cuh);
+// block partials per timeslice, summed by the last block.
 template <bool CB>
 __device__ __forceinline__ void site_obs(const double2 *__restrict__ u, const Lat &l, int par,
                                          const Coord &c, double &e2, double &th) {
     const int op = CB ? (par ^ 1) : 0;
     const int sp = CB ? par : 0;
     const uint32_t si = CB ? (c.L >> 1) : c.L;
-    M3 dA;
-#pragma unroll
-    for (int k = 0; k < 9; k++) dA.e[k] = cz();
+    DivA dA;
+    diva_zero(dA);
 #pragma unroll
     for (int d = 0; d < 3; d++) {
         uint32_t Lb = back_L(l, c, d);
         uint32_t ib = CB ? (Lb >> 1) : Lb;
-        M3 f, r, A1, A2;
+        M3 f, r;
         load_m(u + uidx(l, d, sp, 0, si), l.vh, f);
         load_m(u + uidx(l, d, op, 0, ib), l.vh, r);
-        calc_A(f, A1);
-        calc_A(r, A2);
-#pragma unroll
-        for (int k = 0; k < 9; k++) dA.e[k] = xcadd(dA.e[k], xcsub(A1.e[k], A2.e[k]));
+        diva_add(dA, f, r);
     }
-    // decomposeAlgebraSU3 (SU3_ops.c:1055-1107)
-    const double2 *m = dA.e;
-    double cc[8];
-    cc[0] = xa(m[EL(0, 1)].x, m[EL(1, 0)].x);
-    cc[1] = xa(-m[EL(0, 1)].y, m[EL(1, 0)].y);
-    cc[2] = xs(m[EL(0, 0)].x, m[EL(1, 1)].x);
-    cc[3] = xa(m[EL(0, 2)].x, m[EL(2, 0)].x);
-    cc[4] = xa(-m[EL(0, 2)].y, m[EL(2, 0)].y);
-    cc[5] = xa(m[EL(1, 2)].x, m[EL(2, 1)].x);
-    cc[6] = xa(-m[EL(1, 2)].y, m[EL(2, 1)].y);
-    cc[7] = xd(xs(xa(m[EL(0, 0)].x, m[EL(1, 1)].x), xm(2.0, m[EL(2, 2)].x)), __dsqrt_rn(3.0));
-    double s = 0.0;
-#pragma unroll
-    for (int a = 0; a < 8; a++) s = xa(s, xm(cc[a], cc[a]));
-    e2 = s;
-    // Re Tr(dA dA^dag) = sum_ab |dA_ab|^2 accumulated as the trace of prod3x3
-    double t = 0.0;
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        double2 sa = cz();
-#pragma unroll
-        for (int k = 0; k < 3; k++) sa = xcadd(sa, xcmul(m[EL(a, k)], cconj(m[EL(a, k)])));
-        t = xa(t, sa.x);
-    }
-    th = t;
-}
-
-// block-level deterministic sum of NQ values; result valid in thread 0
-template <int NQ>
-__device__ __forceinline__ void block_sum(double (&v)[NQ]) {
-    __shared__ double sh[NQ][32];
-#pragma unroll
-    for (int q = 0; q < NQ; q++)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
-    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0)
-#pragma unroll
-        for (int q = 0; q < NQ; q++) sh[q][wid] = v[q];
-    __syncthreads();
-    if (wid == 0) {
-        int nw = (blockDim.x + 31) >> 5;
-#pragma unroll
-        for (int q = 0; q < NQ; q++) {
-            v[q] = lane < nw ? sh[q][lane] : 0.0;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
-        }
-    }
-    __syncthreads();
+    diva_densities(dA, e2, th);
 }
 
 // grid (nbx, nt): block bx of slice t sums sites of both parities of slice t.  The
@@ -424,10 +351,20 @@ __device__ __forceinline__ void block_sum(double (&v)[NQ]) {
 // site's backward links are the other parity's, so they are read by a neighbouring
 // thread or a recent block and come from L2, not a second time from DRAM, as they
 // would if one parity's half of the slice were swept before the other's.
-// 128-thread blocks: the six links of a site are all requested at once (~170
-// registers), so three blocks (12 warps) fit on an SM where one 256-thread block did
-__global__ void __launch_bounds__(128) k_obs_partials(const double2 *__restrict__ u, Lat l,
-                                                      double *__restrict__ part, const unsigned *stop) {
+// The six links of a site are requested at once; 128-thread blocks, four to an SM.
+// 32^3 x 64, call to call: 214 us with the reference's operations all carried out (1000
+// FP64 operations per site, most of them scalings and mirror images, see DivA) and a
+// second launch for the sums, 198 us now; its bytes take 139 us at the copy rate.  (223 us
+// marching in z and passing a link's part on to the next site's thread: half the bytes
+// from L2, but its loads wait for one another.)
+//
+// With stop (a stop word; once set, the launch does nothing) and sweep > 0 the proxy (e2 =
+// out[0] / V, or theta = out[1] / 3V, normalised as the host does) below tol sets *stop
+// to sweep: later sweep and observables launches of the stream then do nothing.
+__global__ void __launch_bounds__(128, 4) k_obs(const double2 *__restrict__ u, Lat l, double *__restrict__ part,
+                                                unsigned *__restrict__ ticket, double *__restrict__ out,
+                                                double *__restrict__ slice_out, unsigned *stop, int theta, double tol,
+                                                int sweep) {
     grid_wait();
     if (stop && *(volatile const unsigned *)stop) return;
     const uint32_t t = blockIdx.y;
@@ -449,16 +386,20 @@ __global__ void __launch_bounds__(128) k_obs_partials(const double2 *__restrict_
         v[1] += th;
     }
     block_sum<2>(v);
-    if (threadIdx.x == 0) {
-        size_t o = ((size_t)t * gridDim.x + blockIdx.x) * 2;
-        part[o] = v[0];
-        part[o + 1] = v[1];
+    if (last_block_sum<2>(v, part, ticket, slice_out)) {
+        out[0] = v[0];
+        out[1] = v[1];
+        if (stop && sweep > 0) {
+            const double n3 = (double)l.v, res = theta ? v[1] / (3.0 * n3) : v[0] / n3;
+            if (res <= tol) *stop = (unsigned)sweep;
+        }
     }
 }
 
 // F density: Re Tr of the 3 spatial links at a site (calculateF, gauge_fixing.c:289-337)
-__global__ void __launch_bounds__(256) k_functional_partials(const double2 *__restrict__ u, Lat l,
-                                                             double *__restrict__ part) {
+__global__ void __launch_bounds__(256) k_functional(const double2 *__restrict__ u, Lat l,
+                                                    double *__restrict__ part, unsigned *__restrict__ ticket,
+                                                    double *__restrict__ out) {
     grid_wait();
     const uint32_t t = blockIdx.y;
     const uint32_t vsh = l.cb ? l.vs / 2 : l.vs;
@@ -474,78 +415,25 @@ __global__ void __launch_bounds__(256) k_functional_partials(const double2 *__re
         }
     }
     block_sum<1>(v);
-    if (threadIdx.x == 0) part[(size_t)t * gridDim.x + blockIdx.x] = v[0];
-}
-
-// Sum partials [nt][nbx][nq] per slice in a fixed order, then the slices.
-// out[q] = total, slice_out[t*nq + q] = per slice (optional).
-__global__ void k_finalize(const double *__restrict__ part, int nt, int nbx, int nq, double *__restrict__ out,
-                           double *__restrict__ slice_out, const unsigned *stop) {
-    grid_wait();
-    if (stop && *(volatile const unsigned *)stop) return;
-    __shared__ double acc[4][256];
-    for (int q = 0; q < nq; q++) acc[q][threadIdx.x] = 0.0;
-    for (int t = threadIdx.x; t < nt; t += blockDim.x) {
-        for (int q = 0; q < nq; q++) {
-            double s = 0.0;
-            for (int b = 0; b < nbx; b++) s += part[((size_t)t * nbx + b) * nq + q];
-            if (slice_out) slice_out[(size_t)t * nq + q] = s;
-            acc[q][threadIdx.x] += s;
-        }
-    }
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w)
-            for (int q = 0; q < nq; q++) acc[q][threadIdx.x] += acc[q][threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-        for (int q = 0; q < nq; q++) out[q] = acc[q][0];
+    if (last_block_sum<1>(v, part, ticket, nullptr)) out[0] = v[0];
 }
 
 int obs_blocks_per_slice(const Lat &l) {
-    uint32_t vsh = l.cb ? l.vs / 2 : l.vs;
-    uint32_t n = vsh * l.npar;
-    int nb = (int)((n + 255) / 256);
-    // enough blocks overall to fill the GPU, not more than one per 256 sites
-    int want = (4 * 148 + l.nt - 1) / l.nt;
-    if (nb > want) nb = want;
-    if (nb < 1) nb = 1;
-    return nb;
+    // blocks of 128 sites and more, twelve or so per SM: three or four of them are resident
+    // at a time, so that the last round is a small part of the whole (four per SM left
+    // the second round of two nearly empty)
+    const uint32_t n = (l.vs + 127) / 128, want = (12u * 148u + (uint32_t)l.nt - 1) / (uint32_t)l.nt;
+    return (int)std::min(n, want);
 }
 
-// sums of nbx per-block (e2, theta) partials per timeslice into out[0..1]
-void launch_finalize2(const double *part, const Lat &l, int nbx, double *out, cudaStream_t s, const unsigned *stop) {
-    launch_early(k_finalize, 1, 256, 0, s, part, l.nt, nbx, 2, out, nullptr, stop);
+void launch_obs(const double2 *u, const Lat &l, double *part, unsigned *ticket, double *out, double *slice_out,
+                cudaStream_t s, unsigned *stop, int theta, double tol, int sweep) {
+    launch_early(k_obs, dim3(obs_blocks_per_slice(l), l.nt), 128, 0, s, u, l, part, ticket, out, slice_out, stop, theta,
+                 tol, sweep);
 }
 
-void launch_obs(const double2 *u, const Lat &l, double *part, double *out, double *slice_out, cudaStream_t s,
-                const unsigned *stop) {
-    int nbx = obs_blocks_per_slice(l);
-    launch_early(k_obs_partials, dim3(nbx, l.nt), 128, 0, s, u, l, part, stop);
-    launch_early(k_finalize, 1, 256, 0, s, part, l.nt, nbx, 2, out, slice_out, stop);
-}
-
-// After the observables of half-sweep `sweep`: the proxy (e2 = out[0] / V, or theta =
-// out[1] / 3V, normalised as the host does) below the tolerance sets the stop word to
-// sweep, once; later sweep and observables launches of the stream then do nothing.
-__global__ void k_exact_check(const double *__restrict__ out, double v, int theta, double tol, int sweep,
-                              unsigned *stop) {
-    grid_wait();
-    if (threadIdx.x || blockIdx.x || *(volatile unsigned *)stop) return;
-    const double res = theta ? out[1] / (3.0 * v) : out[0] / v;
-    if (res <= tol) *stop = (unsigned)sweep;
-}
-
-void launch_exact_check(const double *out, const Lat &l, int theta, double tol, int sweep, unsigned *stop,
-                        cudaStream_t s) {
-    launch_early(k_exact_check, 1, 32, 0, s, out, (double)l.v, theta, tol, sweep, stop);
-}
-
-void launch_functional(const double2 *u, const Lat &l, double *part, double *out, cudaStream_t s) {
-    int nbx = obs_blocks_per_slice(l);
-    launch_early(k_functional_partials, dim3(nbx, l.nt), 256, 0, s, u, l, part);
-    launch_early(k_finalize, 1, 256, 0, s, part, l.nt, nbx, 1, out, nullptr, nullptr);
+void launch_functional(const double2 *u, const Lat &l, double *part, unsigned *ticket, double *out, cudaStream_t s) {
+    launch_early(k_functional, dim3(obs_blocks_per_slice(l), l.nt), 256, 0, s, u, l, part, ticket, out);
 }
 
 }  // namespace gfc

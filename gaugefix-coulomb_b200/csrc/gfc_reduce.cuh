@@ -1,0 +1,143 @@
+// gfc_reduce.cuh -- sums over a lattice in one launch: block sums, then the last block to
+// finish adds them up in a fixed order, so the result does not depend on scheduling.
+#pragma once
+#include "gfc_internal.h"
+
+namespace gfc {
+
+// block-level deterministic sum of NQ values; result valid in thread 0
+template <int NQ>
+__device__ __forceinline__ void block_sum(double (&v)[NQ]) {
+    __shared__ double sh[NQ][32];
+#pragma unroll
+    for (int q = 0; q < NQ; q++)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
+    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (lane == 0)
+#pragma unroll
+        for (int q = 0; q < NQ; q++) sh[q][wid] = v[q];
+    __syncthreads();
+    if (wid == 0) {
+        int nw = (blockDim.x + 31) >> 5;
+#pragma unroll
+        for (int q = 0; q < NQ; q++) {
+            v[q] = lane < nw ? sh[q][lane] : 0.0;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
+        }
+    }
+    __syncthreads();
+}
+
+// The block sums v (thread 0) of block (blockIdx.x, timeslice blockIdx.y) go to part
+// [nt][nbx][NQ]; the last block of the grid sums them per timeslice (into slice_out where
+// given), a warp to a timeslice, then the timeslices: true in its thread 0, with the
+// totals in v.  *ticket is zero before and after.
+template <int NQ>
+__device__ __forceinline__ bool last_block_sum(double (&v)[NQ], double *part, unsigned *ticket, double *slice_out) {
+    __shared__ double acc[NQ][32];
+    __shared__ int last;
+    const int nbx = gridDim.x, nt = gridDim.y, tid = threadIdx.x, lane = tid & 31, nw = blockDim.x >> 5;
+    if (tid == 0) {
+        const size_t o = ((size_t)blockIdx.y * nbx + blockIdx.x) * NQ;
+#pragma unroll
+        for (int q = 0; q < NQ; q++) part[o + q] = v[q];
+        __threadfence();
+        last = atomicAdd(ticket, 1u) == (unsigned)(nbx * nt) - 1u;
+    }
+    __syncthreads();
+    if (!last) return false;
+    __threadfence();
+    double a[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; q++) a[q] = 0.0;
+    for (int t = tid >> 5; t < nt; t += nw) {
+        double s[NQ];
+#pragma unroll
+        for (int q = 0; q < NQ; q++) s[q] = 0.0;
+        for (int b = lane; b < nbx; b += 32)
+#pragma unroll
+            for (int q = 0; q < NQ; q++) s[q] += __ldcg(part + ((size_t)t * nbx + b) * NQ + q);
+#pragma unroll
+        for (int q = 0; q < NQ; q++) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s[q] += __shfl_down_sync(0xffffffffu, s[q], o);
+            if (slice_out && lane == 0) slice_out[(size_t)t * NQ + q] = s[q];
+            a[q] += s[q];   // lane 0's
+        }
+    }
+    if (lane == 0)
+#pragma unroll
+        for (int q = 0; q < NQ; q++) acc[q][tid >> 5] = a[q];
+    __syncthreads();
+    if (tid != 0) return false;
+    *ticket = 0;
+#pragma unroll
+    for (int q = 0; q < NQ; q++) {
+        v[q] = 0.0;
+        for (int w = 0; w < nw; w++) v[q] += acc[q][w];
+    }
+    return true;
+}
+
+// The algebra components of div A at a site, in the reference's rounding: added up per
+// direction as calculateA (four_potential.c:35-113, subtractionHermConjTrless3x3
+// SU3_ops.c:322-372) and the divergence do, without the operations that only scale by a
+// power of two (A = -i/2 (...) and the 2 of u - u^dagger on the diagonal), that multiply
+// by zero, or that repeat an entry's mirror image: all of these commute with rounding.
+// With dA_ab = (P - iQ)/2 above the diagonal, (P + iQ)/2 below it and H on it.
+struct DivA {
+    double p[3], q[3], h[3];   // (0,1), (0,2), (1,2); diagonal
+};
+__device__ __forceinline__ void diva_zero(DivA &a) {
+#pragma unroll
+    for (int k = 0; k < 3; k++) a.p[k] = a.q[k] = a.h[k] = 0.0;
+}
+__device__ __forceinline__ void diva_link(const M3 &u, DivA &o) {
+    const double s = xa(xa(u.e[EL(0, 0)].y, u.e[EL(1, 1)].y), u.e[EL(2, 2)].y);
+    const double tr = xdiv_shared(s, 3.0, xrcp(3.0), true);
+#pragma unroll
+    for (int a = 0; a < 3; a++) o.h[a] = xs(u.e[EL(a, a)].y, tr);
+    o.p[0] = xa(u.e[EL(0, 1)].y, u.e[EL(1, 0)].y);
+    o.q[0] = xs(u.e[EL(0, 1)].x, u.e[EL(1, 0)].x);
+    o.p[1] = xa(u.e[EL(0, 2)].y, u.e[EL(2, 0)].y);
+    o.q[1] = xs(u.e[EL(0, 2)].x, u.e[EL(2, 0)].x);
+    o.p[2] = xa(u.e[EL(1, 2)].y, u.e[EL(2, 1)].y);
+    o.q[2] = xs(u.e[EL(1, 2)].x, u.e[EL(2, 1)].x);
+}
+// the forward link f and the backward link r of one direction
+__device__ __forceinline__ void diva_add(DivA &d, const M3 &f, const M3 &r) {
+    DivA a, b;
+    diva_link(f, a);
+    diva_link(r, b);
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        d.p[k] = xa(d.p[k], xs(a.p[k], b.p[k]));
+        d.q[k] = xa(d.q[k], xs(a.q[k], b.q[k]));
+        d.h[k] = xa(d.h[k], xs(a.h[k], b.h[k]));
+    }
+}
+// e2 density sum_a c_a^2 (decomposeAlgebraSU3, SU3_ops.c:1055-1107; gauge_fixing.c:428-438)
+// and theta density Re Tr(dA dA^dagger) (gauge_fixing.c:374-380)
+__device__ __forceinline__ void diva_densities(const DivA &d, double &e2, double &th) {
+    const double c2 = xs(d.h[0], d.h[1]);
+    const double c7 = xd(xs(xa(d.h[0], d.h[1]), xm(2.0, d.h[2])), __dsqrt_rn(3.0));
+    double s = xm(d.p[0], d.p[0]);
+    s = xa(s, xm(d.q[0], d.q[0]));
+    s = xa(s, xm(c2, c2));
+    s = xa(s, xm(d.p[1], d.p[1]));
+    s = xa(s, xm(d.q[1], d.q[1]));
+    s = xa(s, xm(d.p[2], d.p[2]));
+    s = xa(s, xm(d.q[2], d.q[2]));
+    e2 = xa(s, xm(c7, c7));
+    double n[3], m[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        n[k] = xm(0.25, xa(xm(d.p[k], d.p[k]), xm(d.q[k], d.q[k])));
+        m[k] = xm(d.h[k], d.h[k]);
+    }
+    th = xa(xa(xa(xa(m[0], n[0]), n[1]), xa(xa(n[0], m[1]), n[2])), xa(xa(n[1], n[2]), m[2]));
+}
+
+}  // namespace gfc
