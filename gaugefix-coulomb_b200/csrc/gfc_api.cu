@@ -18,6 +18,7 @@
 #include "gfc.h"
 #include "gfc_ctx.h"
 #include "gfc_fast.h"
+#include "gfc_host.h"
 
 namespace gfc {
 
@@ -63,7 +64,6 @@ static void ctx_free(gfc_ctx *c) {
     cudaFree(c->ring);
     for (int k = 0; k < 2; k++) {
         cudaFree(c->dstage[k]);
-        cudaFreeHost(c->hstage[k]);
         if (c->ev_copy[k]) cudaEventDestroy(c->ev_copy[k]);
         if (c->ev_used[k]) cudaEventDestroy(c->ev_used[k]);
     }
@@ -136,7 +136,6 @@ extern "C" int gfc_ctx_create(int ns, int nt, int device, int flags, gfc_ctx **o
         c->stage_bytes = nts * slice_bytes;
         for (int k = 0; k < 2; k++) {
             TRY(cudaMalloc(&c->dstage[k], c->stage_bytes));
-            TRY(cudaMallocHost(&c->hstage[k], c->stage_bytes));
             TRY(cudaEventCreateWithFlags(&c->ev_copy[k], cudaEventDisableTiming));
             TRY(cudaEventCreateWithFlags(&c->ev_used[k], cudaEventDisableTiming));
         }
@@ -176,15 +175,6 @@ extern "C" long long gfc_ctx_kernel_launches(const gfc_ctx *c) { return c ? c->l
 extern "C" void *gfc_ctx_stream(gfc_ctx *c) { return c ? (void *)c->s : nullptr; }
 
 // ------------------------------------------------------- chunked transfers --
-static int is_pinned(const void *p) {
-    cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    return a.type == cudaMemoryTypeHost;
-}
-
 // Host -> device of a raw per-timeslice-ordered array; calls fn(dptr, t0, nts)
 // on the compute stream for each chunk once it is on the device.
 template <typename F>
@@ -197,17 +187,16 @@ static int upload_chunked(gfc_ctx *c, const void *host, size_t bytes_per_slice, 
         uint32_t nts = std::min<uint32_t>(per, l.nt - t0);
         size_t bytes = (size_t)nts * bytes_per_slice;
         const char *src = (const char *)host + (size_t)t0 * bytes_per_slice;
-        // the staging buffer k must be free (its previous transform done)
-        GFC_CHECK(cudaStreamWaitEvent(c->sc, c->ev_used[k], 0));
+        // the staging buffer k must be free (its previous transform done, or copied out)
         if (pinned) {
+            GFC_CHECK(cudaStreamWaitEvent(c->sc, c->ev_used[k], 0));
             GFC_CHECK(cudaMemcpyAsync(c->dstage[k], src, bytes, cudaMemcpyHostToDevice, c->sc));
+            GFC_CHECK(cudaEventRecord(c->ev_copy[k], c->sc));
+            GFC_CHECK(cudaStreamWaitEvent(c->s, c->ev_copy[k], 0));
         } else {
-            GFC_CHECK(cudaEventSynchronize(c->ev_copy[k]));  // host staging k reusable
-            memcpy(c->hstage[k], src, bytes);
-            GFC_CHECK(cudaMemcpyAsync(c->dstage[k], c->hstage[k], bytes, cudaMemcpyHostToDevice, c->sc));
+            int rc = copy_h2d(c->dev, c->dstage[k], src, bytes, c->ev_used[k], c->ev_copy[k]);
+            if (rc) return rc;
         }
-        GFC_CHECK(cudaEventRecord(c->ev_copy[k], c->sc));
-        GFC_CHECK(cudaStreamWaitEvent(c->s, c->ev_copy[k], 0));
         fn(c->dstage[k], t0, nts);
         c->launches++;
         GFC_CHECK(cudaEventRecord(c->ev_used[k], c->s));
@@ -223,42 +212,26 @@ static int download_chunked(gfc_ctx *c, void *host, size_t bytes_per_slice, F fn
     const int pinned = is_pinned(host);
     if (!wait && !pinned) return GFC_ERR_ARG;   // an unfinished copy must land in page-locked memory
     int k = 0;
-    uint32_t pend_t0[2] = {0, 0}, pend_n[2] = {0, 0};
-    int pend[2] = {0, 0};
     for (uint32_t t0 = 0; t0 < (uint32_t)l.nt; t0 += per, k ^= 1) {
         uint32_t nts = std::min<uint32_t>(per, l.nt - t0);
         size_t bytes = (size_t)nts * bytes_per_slice;
+        char *dst = (char *)host + (size_t)t0 * bytes_per_slice;
         // staging k must have been copied out
         GFC_CHECK(cudaStreamWaitEvent(c->s, c->ev_copy[k], 0));
-        if (!pinned && pend[k]) {
-            GFC_CHECK(cudaEventSynchronize(c->ev_copy[k]));
-            memcpy((char *)host + (size_t)pend_t0[k] * bytes_per_slice, c->hstage[k],
-                   (size_t)pend_n[k] * bytes_per_slice);
-            pend[k] = 0;
-        }
         fn(c->dstage[k], t0, nts);
         c->launches++;
         GFC_CHECK(cudaEventRecord(c->ev_used[k], c->s));
-        GFC_CHECK(cudaStreamWaitEvent(c->sc, c->ev_used[k], 0));
-        void *dst = pinned ? (char *)host + (size_t)t0 * bytes_per_slice : c->hstage[k];
-        GFC_CHECK(cudaMemcpyAsync(dst, c->dstage[k], bytes, cudaMemcpyDeviceToHost, c->sc));
-        GFC_CHECK(cudaEventRecord(c->ev_copy[k], c->sc));
-        if (!pinned) {
-            pend[k] = 1;
-            pend_t0[k] = t0;
-            pend_n[k] = nts;
+        if (pinned) {
+            GFC_CHECK(cudaStreamWaitEvent(c->sc, c->ev_used[k], 0));
+            GFC_CHECK(cudaMemcpyAsync(dst, c->dstage[k], bytes, cudaMemcpyDeviceToHost, c->sc));
+            GFC_CHECK(cudaEventRecord(c->ev_copy[k], c->sc));
+        } else {
+            int rc = copy_d2h(c->dev, dst, c->dstage[k], bytes, c->ev_used[k]);
+            if (rc) return rc;
         }
     }
-    if (!wait) {
-        GFC_CHECK(cudaGetLastError());
-        return GFC_OK;
-    }
-    GFC_CHECK(cudaStreamSynchronize(c->sc));
-    for (int j = 0; j < 2; j++)
-        if (pend[j])
-            memcpy((char *)host + (size_t)pend_t0[j] * bytes_per_slice, c->hstage[j],
-                   (size_t)pend_n[j] * bytes_per_slice);
     GFC_CHECK(cudaGetLastError());
+    if (wait) GFC_CHECK(cudaStreamSynchronize(c->sc));
     return GFC_OK;
 }
 

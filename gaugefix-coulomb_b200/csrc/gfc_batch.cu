@@ -33,6 +33,7 @@
 #include "gfc.h"
 #include "gfc_ctx.h"
 #include "gfc_fast_device.cuh"
+#include "gfc_host.h"
 #include "gfc_internal.h"
 
 namespace gfc {
@@ -835,7 +836,7 @@ struct gfc_batch {
     int dev = 0;
     cudaStream_t s = nullptr;
     cudaStream_t s2 = nullptr;       // the odd-ns branch of a captured round
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_host = nullptr;
     int max_slots = 0, max_nt = 0, nslices = 0;
     size_t max_sites = 0, used_sites = 0;
     std::vector<BSlot> hs;          // host copies of the descriptors
@@ -902,6 +903,7 @@ extern "C" int gfc_batch_create(int device, size_t max_sites, int max_slots, int
     BTRY(cudaStreamCreateWithFlags(&b->s2, cudaStreamNonBlocking));
     BTRY(cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming));
     BTRY(cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming));
+    BTRY(cudaEventCreateWithFlags(&b->ev_host, cudaEventDisableTiming));
     BTRY(cudaMalloc(&b->dslots, sizeof(BSlot) * max_slots));
     BTRY(cudaMemset(b->dslots, 0, sizeof(BSlot) * max_slots));
     BTRY(cudaMalloc(&b->state, sizeof(int) * b->nslices));
@@ -986,6 +988,7 @@ extern "C" int gfc_batch_destroy(gfc_batch *b) {
     if (b->s2) cudaStreamDestroy(b->s2);
     if (b->ev_fork) cudaEventDestroy(b->ev_fork);
     if (b->ev_join) cudaEventDestroy(b->ev_join);
+    if (b->ev_host) cudaEventDestroy(b->ev_host);
     delete b;
     return GFC_OK;
 }
@@ -1137,10 +1140,16 @@ extern "C" int gfc_batch_upload(gfc_batch *b, int slot, const void *host, int el
     // the working copies (u64r .. g32, contiguous) are dead outside a fix: >= 576 B per site
     const size_t stage = (size_t)((char *)sl.part - (char *)sl.u64r);
     const uint32_t per = (uint32_t)std::max<size_t>(1, stage / per_slice);
+    const int pageable = is_pageable(host);
     for (uint32_t t0 = 0; t0 < (uint32_t)l.nt; t0 += per) {
         uint32_t n = std::min<uint32_t>(per, l.nt - t0);
-        GFC_CHECK(cudaMemcpyAsync(sl.u64r, (const char *)host + (size_t)t0 * per_slice, n * per_slice,
-                                  cudaMemcpyHostToDevice, b->s));
+        const char *src = (const char *)host + (size_t)t0 * per_slice;
+        if (pageable) {
+            GFC_CHECK(cudaEventRecord(b->ev_host, b->s));
+            if ((rc = copy_h2d(b->dev, sl.u64r, src, n * per_slice, b->ev_host))) return rc;
+        } else {
+            GFC_CHECK(cudaMemcpyAsync(sl.u64r, src, n * per_slice, cudaMemcpyHostToDevice, b->s));
+        }
         // byte swap, precision, layout and reunitarisation in one pass
         launch_load_links(sl.u64r, elem_bytes, byteswap, l, t0, n, sl.u, sl.ut, b->s, 1, b->status);
     }
@@ -1475,6 +1484,18 @@ extern "C" int gfc_batch_plaquette(gfc_batch *b, int slot, double *spatial, doub
 }
 
 namespace gfc {
+// staged raw output to host memory, after the work queued on st so far; the copy to
+// ordinary memory is done on return, one to page-locked memory is queued on st
+static int copy_out(gfc_batch *b, char *host, const void *dev, size_t bytes, int pageable, cudaStream_t st) {
+    if (!pageable) {
+        GFC_CHECK(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, st));
+        return GFC_OK;
+    }
+    // the stream's own wait, not an event: the result thread and the caller may both be here
+    GFC_CHECK(cudaStreamSynchronize(st));
+    return copy_d2h(b->dev, host, dev, bytes);
+}
+
 // G of a finalised slot to host memory on stream `st` (the caller's stream: the
 // request server downloads on its own stream while rounds run on the batch's)
 int batch_download_gt_on(gfc_batch *b, int slot, void *host, int elem_bytes, int byteswap, cudaStream_t st) {
@@ -1493,11 +1514,11 @@ int batch_download_gt_on(gfc_batch *b, int slot, void *host, int elem_bytes, int
     // the working copies (u64r .. g32, contiguous) are dead outside a fix: >= 576 B per site
     const size_t stage = (size_t)((char *)sl.part - (char *)sl.u64r);
     const uint32_t per = (uint32_t)std::max<size_t>(1, stage / per_slice);
+    const int pageable = is_pageable(host);
     for (uint32_t t0 = 0; t0 < (uint32_t)l.nt; t0 += per) {
         uint32_t n = std::min<uint32_t>(per, l.nt - t0);
         launch_store_gt(sl.g, l, t0, n, elem_bytes, byteswap, sl.u64r, st);
-        GFC_CHECK(cudaMemcpyAsync((char *)host + (size_t)t0 * per_slice, sl.u64r, n * per_slice,
-                                  cudaMemcpyDeviceToHost, st));
+        if ((rc = copy_out(b, (char *)host + (size_t)t0 * per_slice, sl.u64r, n * per_slice, pageable, st))) return rc;
     }
     GFC_CHECK(cudaStreamSynchronize(st));
     return GFC_OK;
@@ -1539,11 +1560,12 @@ extern "C" int gfc_batch_download_links(gfc_batch *b, int slot, void *host, int 
     // the working copies (u64r .. g32, contiguous) are dead outside a fix: >= 576 B per site
     const size_t stage = (size_t)((char *)sl.part - (char *)sl.u64r);
     const uint32_t per = (uint32_t)std::max<size_t>(1, stage / per_slice);
+    const int pageable = is_pageable(host);
     for (uint32_t t0 = 0; t0 < (uint32_t)l.nt; t0 += per) {
         uint32_t n = std::min<uint32_t>(per, l.nt - t0);
         launch_store_links(sl.u, sl.ut, l, t0, n, elem_bytes, byteswap, sl.u64r, b->s);
-        GFC_CHECK(cudaMemcpyAsync((char *)host + (size_t)t0 * per_slice, sl.u64r, n * per_slice,
-                                  cudaMemcpyDeviceToHost, b->s));
+        if ((rc = copy_out(b, (char *)host + (size_t)t0 * per_slice, sl.u64r, n * per_slice, pageable, b->s)))
+            return rc;
     }
     GFC_CHECK(cudaStreamSynchronize(b->s));
     return GFC_OK;

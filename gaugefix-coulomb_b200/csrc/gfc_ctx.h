@@ -34,7 +34,6 @@ struct gfc_ctx {
     // chunked I/O staging
     size_t stage_bytes = 0;
     void *dstage[2] = {nullptr, nullptr};
-    void *hstage[2] = {nullptr, nullptr};
     cudaEvent_t ev_copy[2] = {nullptr, nullptr}, ev_used[2] = {nullptr, nullptr};
     cudaEvent_t ev_a = nullptr, ev_b = nullptr, ev_c = nullptr, ev_d = nullptr;
     unsigned *tickets = nullptr;  // [nt + 2]: per-slice and global tickets, stop word

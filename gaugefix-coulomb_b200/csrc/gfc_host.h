@@ -1,0 +1,20 @@
+// gfc_host.h -- copies between device memory and ordinary (pageable) host memory.
+#pragma once
+#include <cuda_runtime.h>
+#include <stddef.h>
+
+namespace gfc {
+
+// 1 if p is page-locked host memory
+int is_pinned(const void *p);
+// 1 if p is ordinary host memory, which copy_h2d / copy_d2h take
+int is_pageable(const void *p);
+// Copy to or from ordinary host memory on `device`; the data is there on return.  The
+// device side is used after the work recorded in a and b (events; may be null).
+// Returns a GFC_* code.
+int copy_h2d(int device, void *dev, const void *host, size_t bytes, cudaEvent_t a = nullptr, cudaEvent_t b = nullptr);
+int copy_d2h(int device, void *host, const void *dev, size_t bytes, cudaEvent_t a = nullptr, cudaEvent_t b = nullptr);
+// memcpy on several threads
+void copy_host(void *dst, const void *src, size_t bytes);
+
+}  // namespace gfc

@@ -18,12 +18,14 @@
 #include <cstring>
 #include <deque>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <thread>
 #include <vector>
 
 #include "gfc.h"
 #include "gfc_ctx.h"
+#include "gfc_host.h"
 
 namespace {
 
@@ -40,7 +42,8 @@ struct Request {
     int synth = 0;           // 1: seeded synthetic links built on the device at admission
     uint64_t seed = 0;
     double scale = 0;
-    std::vector<char> raw;   // uploaded links (copied at submit), elem_bytes / byteswap below
+    std::unique_ptr<char, decltype(&free)> raw{nullptr, &free};   // uploaded links (copied at
+                             // submit), elem_bytes / byteswap below
     int elem_bytes = 8, byteswap = 0;
     double t_submit = 0, t_admit = 0, t_done = 0;
     int slot = -1;
@@ -263,7 +266,16 @@ extern "C" int gfc_server_submit(gfc_server *s, int ns, int nt, const void *link
     r.scale = scale;
     r.elem_bytes = elem_bytes;
     r.byteswap = byteswap;
-    if (links) r.raw.assign((const char *)links, (const char *)links + V * 4 * 18 * elem_bytes);
+    if (links) {
+        // not zeroed first, and its pages first touched by several threads
+        const size_t bytes = V * 4 * 18 * (size_t)elem_bytes;
+        r.raw.reset((char *)malloc(bytes));
+        if (!r.raw) {
+            set_error("host memory for a request of %zu bytes", bytes);
+            return GFC_ERR_NOMEM;
+        }
+        copy_host(r.raw.get(), links, bytes);
+    }
     r.t_submit = now_s();
     std::lock_guard<std::mutex> lk(s->mu);
     r.id = s->next_id++;
@@ -311,10 +323,10 @@ extern "C" int gfc_server_step(gfc_server *s, const gfc_params *p, const gfc_opt
         }
         if (rc) return rc;
         rc = r->synth ? gfc_batch_synth(s->b, slot, r->seed, r->scale)
-                      : gfc_batch_upload(s->b, slot, r->raw.data(), r->elem_bytes, r->byteswap);
+                      : gfc_batch_upload(s->b, slot, r->raw.get(), r->elem_bytes, r->byteswap);
         if (!rc) rc = gfc_batch_activate(s->b, slot, r->precision);
         if (rc) return rc;
-        std::vector<char>().swap(r->raw);
+        r->raw.reset();
         {
             std::lock_guard<std::mutex> lk(s->mu);
             r->slot = slot;
@@ -424,7 +436,7 @@ extern "C" int gfc_server_fetch(gfc_server *s, int64_t id, void *gt, int elem_by
     if (r.err) return r.err;
     if (gt) {
         if (elem_bytes == 8) {
-            memcpy(gt, r.gt, r.gt_n * sizeof(double));
+            copy_host(gt, r.gt, r.gt_n * sizeof(double));
         } else {
             float *f = (float *)gt;
             for (size_t k = 0; k < r.gt_n; k++) f[k] = (float)r.gt[k];
