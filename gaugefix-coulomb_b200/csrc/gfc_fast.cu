@@ -61,6 +61,7 @@ struct SweepArgs {
     double tol_sum;     // stop when post(sweep-1) + pre(sweep) <= tol_sum
     int test;           // 1: hist holds post(sweep-1) of this run, so the stop test applies
     unsigned *status;
+    int keep;           // timeslices left in L2 from one half-sweep to the next, 0: no hints
     int proj;           // 1: project the links written onto SU(3) (reunitarisation folded in;
                         // honoured by the fully staged two-row shapes, see links_fold_reunit)
 };
@@ -198,7 +199,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_sweep_fast(typename S::V *__res
     if (a.track) fused_reduce<BLOCK>(a, pre, post, sh, last);
 }
 
-template <class S, int BLOCK, int MINB, bool SG, int NST, bool PROJ = false>
+template <class S, int BLOCK, int MINB, bool SG, int NST, bool PROJ = false, bool HINT = false>
 __global__ void __launch_bounds__(BLOCK, MINB) k_sweep_staged(typename S::V *__restrict__ u,
                                                               typename S::V *__restrict__ g, SweepArgs a) {
     extern __shared__ __align__(16) unsigned char staged_smem[];
@@ -210,9 +211,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_sweep_staged(typename S::V *__r
     const uint32_t off = blockIdx.x * BLOCK + threadIdx.x;
     double pre = 0.0, post = 0.0;
     if (off < vsh)
-        fast_site_staged<S, BLOCK, SG, NST, true, PROJ>(u, g, l, a.par, (a.t0 + blockIdx.y) * vsh + off, (T)a.omega,
-                                                        a.hits, a.track, pre, post, (typename S::V *)staged_smem,
-                                                        a.status);
+        fast_site_staged<S, BLOCK, SG, NST, true, PROJ, HINT>(
+            u, g, l, a.par, (a.t0 + blockIdx.y) * vsh + off, (T)a.omega, a.hits, a.track, pre, post,
+            (typename S::V *)staged_smem, a.status,
+            HINT ? l2_policy((int)(a.t0 + blockIdx.y) < a.keep) : 0);
     if (a.track) {
         // the reduction's scratch reuses the staging buffer: it has no static shared
         // memory, so 32-site blocks fit 12 to an SM; every thread is done with its
@@ -462,20 +464,25 @@ static void launch_staged(dim3 grid, cudaStream_t st, typename S::V *u, typename
     constexpr size_t bytes = staged_bytes<S>(sh.block, sh.sg, sh.nst);
     static_assert(bytes <= 227 * 1024, "staged tile exceeds shared memory");
     static_assert(sh.block >= MIN_BLOCK, "block partial buffers are sized for MIN_BLOCK");
-    auto kern = k_sweep_staged<S, sh.block, sh.minb, (bool)sh.sg, sh.nst>;
-    static std::atomic<unsigned long long> done{0};
-    smem_attr_once(done, kern, bytes);
     grid.x = ((a.l.vs >> 1) + sh.block - 1) / sh.block;
-    if constexpr ((std::is_same<S, S64R>::value || std::is_same<S, S32>::value) && sh.nst == 6) {
-        if (a.proj) {
-            auto kp = k_sweep_staged<S, sh.block, sh.minb, (bool)sh.sg, sh.nst, true>;
-            static std::atomic<unsigned long long> done_p{0};
-            smem_attr_once(done_p, kp, bytes);
-            launch_early(kp, grid, sh.block, bytes, st, u, g, a);
-            return;
-        }
+    auto launch = [&](auto kern, std::atomic<unsigned long long> &done) {
+        smem_attr_once(done, kern, bytes);
+        launch_early(kern, grid, sh.block, bytes, st, u, g, a);
+    };
+    static std::atomic<unsigned long long> done[4];
+    if constexpr (sh.nst == 6) {
+        constexpr bool sg = sh.sg;
+        if (a.proj && a.keep)
+            launch(k_sweep_staged<S, sh.block, sh.minb, sg, 6, true, true>, done[3]);
+        else if (a.proj)
+            launch(k_sweep_staged<S, sh.block, sh.minb, sg, 6, true, false>, done[2]);
+        else if (a.keep)
+            launch(k_sweep_staged<S, sh.block, sh.minb, sg, 6, false, true>, done[1]);
+        else
+            launch(k_sweep_staged<S, sh.block, sh.minb, sg, 6, false, false>, done[0]);
+    } else {
+        launch(k_sweep_staged<S, sh.block, sh.minb, (bool)sh.sg, sh.nst>, done[0]);
     }
-    launch_early(kern, grid, sh.block, bytes, st, u, g, a);
 }
 
 // Whether a half-sweep launched with SweepArgs::proj projects the links it writes
@@ -522,6 +529,19 @@ static void dispatch_fast(int v, dim3 grid, cudaStream_t st, typename S::V *u, t
     }
 }
 
+// Timeslices whose fields a sweep leaves in L2 for the next half-sweep (l2_policy), 0: the
+// sweep carries no hints.  80 MB of L2's 126 (40 to 100 MB measured within 1 % of one
+// another) are worth it on lattices of up to 300 MB: with hints against without, FP32 28^3 x
+// 48 (202 MB) 60.0 and 61.9 us per half-sweep, FP64 24^3 x 48 (255 MB) 72.3 and 74.4, but
+// FP64 28^3 x 48 (404 MB) 118.7 and 116.6, 32^3 x 64 (805 MB) 222 and 219; and on 16^3 x 32,
+// which L2 holds whole, 13.9 and 13.7.
+template <class S>
+static int keep_slices(const Lat &l, int nsl) {
+    const size_t slice = (size_t)l.vs * 4 * S::BYTES, all = slice * l.nt, budget = (size_t)80 << 20;
+    if (nsl >= 0 || all <= budget || all > (size_t)300 << 20) return 0;
+    return std::max(1, (int)(budget / slice));
+}
+
 // One half-sweep of timeslices [t0, t0 + nsl) (all slices by default).
 template <class S>
 static void launch_fast(gfc_ctx *c, typename S::V *u, typename S::V *g, int sweep, double omega, unsigned hits,
@@ -548,6 +568,7 @@ static void launch_fast(gfc_ctx *c, typename S::V *u, typename S::V *g, int swee
     a.tol_sum = tol_sum;
     a.test = test;
     a.status = c->dstatus;
+    a.keep = keep_slices<S>(l, nsl);
     a.proj = proj;
     const int v = sizeof(typename S::T) == 8 ? c->shape_fast64 : c->shape_fast32;
     dispatch_fast<S>(v, dim3(0, nsl < 0 ? l.nt : nsl), c->s, u, g, a);
@@ -1169,6 +1190,7 @@ extern "C" int gfc_ctx_autotune(gfc_ctx *c, int which, double *times_out) {
         a.stop = nullptr;
         a.tol_sum = 0.0;
         a.status = c->dstatus;
+        a.keep = 0;
         return a;
     };
     if (which & 1) {

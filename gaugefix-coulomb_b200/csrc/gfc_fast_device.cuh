@@ -655,16 +655,64 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
+// ------------------------------------------------------ L2 cache hints --
+// The fields of a lattice larger than L2 are swept from end to end, half-sweep after
+// half-sweep, so with every line treated alike each is evicted before it is read again.
+// The first timeslices are marked "evict last" and the others "evict first": the first
+// ones stay in L2 from one half-sweep to the next (FP32 24^3 x 48, 127 MB: 39.1 -> 34.9 us
+// per half-sweep; FP64 20^3 x 40, 123 MB: 36.6 -> 31.5).  See keep_slices for where it pays.
+__device__ __forceinline__ uint64_t l2_policy(bool keep) {
+    uint64_t a, b;
+    asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;\n" : "=l"(a));
+    asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;\n" : "=l"(b));
+    return keep ? a : b;
+}
+template <bool HINT, typename V>
+__device__ __forceinline__ void cp_async16_hint(V *smem, const V *gmem, uint64_t policy) {
+    if constexpr (HINT) {
+        const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+        asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "l"(policy)
+                     : "memory");
+    } else {
+        cp_async16(smem, gmem);
+    }
+}
+template <bool HINT>
+__device__ __forceinline__ void st_hint(double2 *p, double2 v, uint64_t policy) {
+    if constexpr (HINT)
+        asm volatile("st.global.L2::cache_hint.v2.f64 [%0], {%1, %2}, %3;\n" ::"l"(p), "d"(v.x), "d"(v.y), "l"(policy)
+                     : "memory");
+    else
+        *p = v;
+}
+template <bool HINT>
+__device__ __forceinline__ void st_hint(float4 *p, float4 v, uint64_t policy) {
+    if constexpr (HINT)
+        asm volatile("st.global.L2::cache_hint.v4.f32 [%0], {%1, %2, %3, %4}, %5;\n" ::"l"(p), "f"(v.x), "f"(v.y),
+                     "f"(v.z), "f"(v.w), "l"(policy)
+                     : "memory");
+    else
+        *p = v;
+}
+// rows 0 and 1 into two-row storage S
+template <class S, bool HINT>
+__device__ __forceinline__ void store_hint(typename S::V *p, size_t st, const Mt<typename S::T> &m, uint64_t policy) {
+    typename S::V v[S::NS];
+    S::store(v, 1, m);
+#pragma unroll
+    for (int e = 0; e < S::NS; e++) st_hint<HINT>(p + (size_t)e * st, v[e], policy);
+}
+
 // up . f (forward link) or r . up^dagger (backward link) from a staged copy `src`
 // (stride sst) to global `dst` (stride st); rows 0 and 1 are stored, row 2 only
 // enters e2.  PROJ: the link is projected onto SU(3) before it is stored (a
 // reunitarisation folded into the half-sweep).  projectSU3 reads rows 0 and 1 only,
 // so the stored rows are those a separate pass would leave; a null row sets the
 // status bit as that pass does.
-template <class S, bool FWD, bool PROJ = false>
+template <class S, bool FWD, bool PROJ = false, bool HINT = false>
 __device__ __forceinline__ void apply_staged(const typename S::V *src, int sst, typename S::V *__restrict__ dst,
                                              size_t st, const Mt<typename S::T> &up, int track, double (&cc)[8],
-                                             unsigned *status = nullptr) {
+                                             uint64_t policy, unsigned *status = nullptr) {
     using T = typename S::T;
     using C = typename CT<T>::t;
     const double sg = FWD ? 1.0 : -1.0;
@@ -704,7 +752,7 @@ __device__ __forceinline__ void apply_staged(const typename S::V *src, int sst, 
         }
         if (!fproject(o) && status) atomicOr(status, GFC_STATUS_PROJECT_FAIL);
 #pragma unroll
-        for (int e = 0; e < 6; e++) dst[(size_t)e * st] = o.e[e];
+        for (int e = 0; e < 6; e++) st_hint<HINT>(dst + (size_t)e * st, o.e[e], policy);
     } else if constexpr (S::ROWWISE) {
         // one output row at a time; operands are read back from shared memory as
         // needed rather than held (row 2 of the link is rebuilt from rows 0 and 1)
@@ -734,7 +782,7 @@ __device__ __forceinline__ void apply_staged(const typename S::V *src, int sst, 
                     v = fmac_conj(v, m2, up.e[EL(j, 2)]);
                 }
                 o[j] = v;
-                if (r < 2) dst[(size_t)(3 * r + j) * st] = v;
+                if (r < 2) st_hint<HINT>(dst + (size_t)(3 * r + j) * st, v, policy);
             }
             if (track) {
                 if (r == 0) acc_row<0>(cc, o[0], o[1], o[2], sg);
@@ -774,7 +822,7 @@ __device__ __forceinline__ void apply_staged(const typename S::V *src, int sst, 
         if constexpr (PROJ) {
             if (!fproject(o) && status) atomicOr(status, GFC_STATUS_PROJECT_FAIL);
         }
-        S::store(dst, st, o);   // rows 0 and 1
+        store_hint<S, HINT>(dst, st, o, policy);   // rows 0 and 1
     }
 }
 
@@ -786,12 +834,14 @@ __device__ __forceinline__ void apply_staged(const typename S::V *src, int sst, 
 // thread x at sm[(m * NS + e) * BLOCK + x] (m = 2d forward, 2d+1 backward link of
 // direction d, m = NST for G).  Two-row storage only.  CB = false: odd ns (one parity
 // slot, i = the site's lexicographic index, its place in the fields odd_slot of it).
-// PROJ: the six links written are projected onto SU(3) first (apply_staged).
-template <class S, int BLOCK, bool SG, int NST = 6, bool CB = true, bool PROJ = false>
+// PROJ: the six links written are projected onto SU(3) first (apply_staged).  HINT: staged
+// loads and stores carry the L2 policy given.
+template <class S, int BLOCK, bool SG, int NST = 6, bool CB = true, bool PROJ = false, bool HINT = false>
 __device__ __forceinline__ void fast_site_staged(typename S::V *__restrict__ u, typename S::V *__restrict__ g,
                                                  const Lat &l, int par, uint32_t i, typename S::T omega,
                                                  unsigned hits, int track, double &pre, double &post,
-                                                 typename S::V *sm, unsigned *status = nullptr) {
+                                                 typename S::V *sm, unsigned *status = nullptr,
+                                                 uint64_t policy = 0) {
     using T = typename S::T;
     using C = typename CT<T>::t;
     using V = typename S::V;
@@ -813,14 +863,14 @@ __device__ __forceinline__ void fast_site_staged(typename S::V *__restrict__ u, 
         const V *r = u + su_idx<S>(l, d, op, ib[d]);
 #pragma unroll
         for (int e = 0; e < S::NS; e++) {
-            cp_async16(my + ((2 * d) * S::NS + e) * BLOCK, f + (size_t)e * l.vh);
-            cp_async16(my + ((2 * d + 1) * S::NS + e) * BLOCK, r + (size_t)e * l.vh);
+            cp_async16_hint<HINT>(my + ((2 * d) * S::NS + e) * BLOCK, f + (size_t)e * l.vh, policy);
+            cp_async16_hint<HINT>(my + ((2 * d + 1) * S::NS + e) * BLOCK, r + (size_t)e * l.vh, policy);
         }
     }
     if (SG) {
         const V *gp = g + sg_idx<S>(l, par, i);
 #pragma unroll
-        for (int e = 0; e < S::NS; e++) cp_async16(my + (NST * S::NS + e) * BLOCK, gp + (size_t)e * l.vh);
+        for (int e = 0; e < S::NS; e++) cp_async16_hint<HINT>(my + (NST * S::NS + e) * BLOCK, gp + (size_t)e * l.vh, policy);
     }
     cp_async_wait_all();
 
@@ -860,7 +910,7 @@ __device__ __forceinline__ void fast_site_staged(typename S::V *__restrict__ u, 
         else
             S::load(g + sg_idx<S>(l, par, i), l.vh, m);
         fprod_left<S>(up, m, o);
-        S::store(g + sg_idx<S>(l, par, i), l.vh, o);
+        store_hint<S, HINT>(g + sg_idx<S>(l, par, i), l.vh, o, policy);
     }
     double cc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if constexpr (ND == 3) {
@@ -871,19 +921,19 @@ __device__ __forceinline__ void fast_site_staged(typename S::V *__restrict__ u, 
 #pragma unroll 1
         for (int d = 0; d < 3; d++) {
             const uint32_t b = d == 0 ? ib[0] : (d == 1 ? ib[1] : ib[2]);
-            apply_staged<S, true, PROJ>(my + (2 * d) * S::NS * BLOCK, BLOCK, u + su_idx<S>(l, d, par, i), l.vh,
-                                        up, track_links, cc, status);
-            apply_staged<S, false, PROJ>(my + (2 * d + 1) * S::NS * BLOCK, BLOCK, u + su_idx<S>(l, d, op, b), l.vh,
-                                         up, track_links, cc, status);
+            apply_staged<S, true, PROJ, HINT>(my + (2 * d) * S::NS * BLOCK, BLOCK, u + su_idx<S>(l, d, par, i), l.vh,
+                                        up, track_links, cc, policy, status);
+            apply_staged<S, false, PROJ, HINT>(my + (2 * d + 1) * S::NS * BLOCK, BLOCK, u + su_idx<S>(l, d, op, b), l.vh,
+                                         up, track_links, cc, policy, status);
         }
     } else
 #pragma unroll
     for (int d = 0; d < 3; d++) {
         if (d < ND) {
-            apply_staged<S, true>(my + (2 * d) * S::NS * BLOCK, BLOCK, u + su_idx<S>(l, d, par, i), l.vh, up,
-                                  track_links, cc);
-            apply_staged<S, false>(my + (2 * d + 1) * S::NS * BLOCK, BLOCK, u + su_idx<S>(l, d, op, ib[d]), l.vh,
-                                   up, track_links, cc);
+            apply_staged<S, true, false, HINT>(my + (2 * d) * S::NS * BLOCK, BLOCK, u + su_idx<S>(l, d, par, i), l.vh, up,
+                                  track_links, cc, policy);
+            apply_staged<S, false, false, HINT>(my + (2 * d + 1) * S::NS * BLOCK, BLOCK, u + su_idx<S>(l, d, op, ib[d]), l.vh,
+                                   up, track_links, cc, policy);
         } else {
             apply_forward<S>(u + su_idx<S>(l, d, par, i), l.vh, up, track_links, cc);
             apply_backward<S>(u + su_idx<S>(l, d, op, ib[d]), l.vh, up, track_links, cc);
