@@ -170,6 +170,249 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_sweep_exact_staged(double2 *__r
     site_update_exact_staged<BLOCK>(u, g, l, par, c, omega, hits, (double2 *)exact_stage);
 }
 
+// The same update with a site on three lanes, one to a column of its matrices: a small
+// lattice has a few warps per SM, and a half-sweep takes as long as one warp's chain of
+// instructions (3700 FP64 operations per site and thread).  Per half-sweep, a thread and
+// three lanes to a site: 4^3 x 8 9.2 and 6.6 us, 8^3 x 16 10.0 and 7.0, 12^3 x 24 (four of the
+// former's warps per SM) 16.4 and 13.4, but 16^3 x 32 (fourteen) 27.5 and 34.3, where the
+// scalars done three times over count; odd ns: 9^3 x 8 37.8 and 28.2, 13^3 x 26 52 and 43,
+// 15^3 x 32 53 and 64.  A column of
+// a product needs the left factor whole and the right one's column, so each lane does a
+// third of w, of the inverse, of the rotations and of the seven products, and the scalars
+// (determinant, square roots, norms) in full; what it needs of the other columns passes
+// through shared memory.  Every entry is computed from the same operands in the same order
+// as by one thread: the same bits.
+//
+// A warp takes 10 sites: lane = 3 * site + column (lanes 30, 31 repeat site 9's first two
+// and store nothing).  Shared memory of a warp, in 16-byte entries: the six links of its
+// sites, entry e of link m of site s at (m * 9 + e) * 10 + s, then one matrix of scratch.
+constexpr int COL_SITES = 10;
+constexpr int COL_UNITS = 63 * COL_SITES;
+__device__ __forceinline__ void col_prod(const M3 &a, const double2 (&b)[3], double2 (&t)[3]) {
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+        double2 s = cz();
+#pragma unroll
+        for (int k = 0; k < 3; k++) s = xcadd(s, xcmul(a.e[EL(r, k)], b[k]));
+        t[r] = s;
+    }
+}
+// sum of the three lanes' |v|^2 in column order (xnormalize), v scaled; -1 for a null row
+__device__ __forceinline__ int col_normalize(double2 &v, int l0) {
+    const double h = xhypot(v.x, v.y), hh = xm(h, h);
+    double r = xa(0.0, __shfl_sync(0xffffffffu, hh, l0));
+    r = xa(r, __shfl_sync(0xffffffffu, hh, l0 + 1));
+    r = xa(r, __shfl_sync(0xffffffffu, hh, l0 + 2));
+    if (r == 0.0) return -1;
+    r = xrcp(__dsqrt_rn(r));
+    v = make_double2(xm(v.x, r), xm(v.y, r));
+    return 0;
+}
+// conj(u[a] v[b] - u[b] v[a])
+__device__ __forceinline__ double2 col_cross(double2 ua, double2 ub, double2 va, double2 vb) {
+    return cconj(xcsub(xcmul(ua, vb), xcmul(ub, va)));
+}
+template <int A, int B>
+__device__ __forceinline__ void col_sub_los_alamos(double2 (&w)[3], double2 *X, int c) {
+    constexpr int N = COL_SITES;
+    X[(3 * A + c) * N] = w[A];
+    X[(3 * B + c) * N] = w[B];
+    __syncwarp();
+    const double2 aa = X[(3 * A + A) * N], ab = X[(3 * A + B) * N], ba = X[(3 * B + A) * N], bb = X[(3 * B + B) * N];
+    __syncwarp();
+    double k0 = xa(aa.x, bb.x);
+    double k1 = -xa(ab.y, ba.y);
+    double k2 = -xs(ab.x, ba.x);
+    double k3 = -xs(aa.y, bb.y);
+    const double det = xa(xa(xa(xa(0.0, xm(k0, k0)), xm(k1, k1)), xm(k2, k2)), xm(k3, k3));
+    if (det == 0.0) return;
+    const double inv = xrcp(__dsqrt_rn(det));
+    k0 = xm(inv, k0);
+    k1 = xm(inv, k1);
+    k2 = xm(inv, k2);
+    k3 = xm(inv, k3);
+    const double2 ga = w[A], gb = w[B];
+    w[A] = xcadd(xcmul(make_double2(k0, k3), ga), xcmul(make_double2(k2, k1), gb));
+    w[B] = xcadd(xcmul(make_double2(-k2, k1), ga), xcmul(make_double2(k0, -k3), gb));
+}
+// The j-th site of a launch: the checkerboard's (CB), or one of a boundary level of odd ns
+// (lexicographic layout); false past the last one (a valid site is given all the same).
+template <bool CB>
+__device__ __forceinline__ bool col_site(const Lat &l, int sweep, int level, uint32_t j, Coord &c) {
+    if (CB) {
+        const bool on = j < l.vh;
+        c = coord_cb(l, sweep & 1, on ? j : l.vh - 1);
+        return on;
+    }
+    const uint32_t n = odd_level_count(l, level), t = j / n;
+    uint32_t off = 0;
+    const bool on = t < (uint32_t)l.nt && odd_level_site(l, sweep & 1, t, level, j - t * n, off);
+    c = coord_lex(l, on ? t * l.vs + off : 0);
+    return on;
+}
+template <bool CB>
+__global__ void __launch_bounds__(32, 16) k_sweep_exact_cols(double2 *__restrict__ u, double2 *__restrict__ g, Lat l,
+                                                             int sweep, int level, double omega, unsigned hits,
+                                                             const unsigned *stop) {
+    extern __shared__ __align__(16) unsigned char cols_stage[];
+    constexpr int N = COL_SITES;
+    const int lane = threadIdx.x, par = CB ? sweep & 1 : 0, op = CB ? par ^ 1 : 0;
+    double2 *sm = (double2 *)cols_stage;
+    const uint32_t j0 = blockIdx.x * N;
+    grid_wait();
+    if (stop && *(volatile const unsigned *)stop) return;
+    // copy: a lane takes a row of the six links of one site
+    {
+        const int ls = lane % N, q = lane / N;
+        if (q < 3) {
+            Coord cc;
+            col_site<CB>(l, sweep, level, j0 + ls, cc);
+            const uint32_t i = CB ? cc.L >> 1 : cc.L;
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                const uint32_t Lb = back_L(l, cc, d);
+                const double2 *f = u + uidx(l, d, par, 3 * q, i);
+                const double2 *r = u + uidx(l, d, op, 3 * q, CB ? Lb >> 1 : Lb);
+#pragma unroll
+                for (int e = 0; e < 3; e++) {
+                    const unsigned sf = (unsigned)__cvta_generic_to_shared(sm + ((2 * d) * 9 + 3 * q + e) * N + ls);
+                    const unsigned sr = (unsigned)__cvta_generic_to_shared(sm + ((2 * d + 1) * 9 + 3 * q + e) * N + ls);
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sf), "l"(f + (size_t)e * l.vh) : "memory");
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sr), "l"(r + (size_t)e * l.vh) : "memory");
+                }
+            }
+        }
+    }
+    // compute: a lane has column c of site s
+    const int sl = lane < 30 ? lane : lane - 3, s = sl / 3, c = sl - 3 * s, l0 = 3 * s;
+    const int ca = c == 2 ? 0 : c + 1, cb = c == 0 ? 2 : c - 1;   // the columns after it, cyclically
+    Coord cs;
+    const bool keep = col_site<CB>(l, sweep, level, j0 + s, cs) && lane < 30;
+    const uint32_t si = CB ? cs.L >> 1 : cs.L;
+    uint32_t ib[3];
+#pragma unroll
+    for (int d = 0; d < 3; d++) ib[d] = CB ? back_L(l, cs, d) >> 1 : back_L(l, cs, d);
+#pragma unroll
+    for (int r = 0; r < 3; r++) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(g + gidx(l, par, 3 * r + c, si)));
+    sm += s;
+    double2 *X = sm + 54 * N;
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncwarp();
+    double2 w[3] = {cz(), cz(), cz()};
+#pragma unroll 1
+    for (int d = 0; d < 3; d++)
+#pragma unroll
+        for (int r = 0; r < 3; r++)
+            w[r] = xcadd(w[r], xcadd(sm[((2 * d) * 9 + 3 * r + c) * N], cconj(sm[((2 * d + 1) * 9 + 3 * c + r) * N])));
+    // column c of the inverse (xinverse): from rows c + 1 and c + 2 of w
+#pragma unroll
+    for (int r = 0; r < 3; r++) X[(3 * r + c) * N] = w[r];
+    __syncwarp();
+    double2 v[3];
+    double dre;
+    {
+        double2 t = xcmul(w[0], xcsub(xcmul(X[(3 + ca) * N], X[(6 + cb) * N]), xcmul(X[(3 + cb) * N], X[(6 + ca) * N])));
+        double2 t0, t1, t2;
+        t0.x = __shfl_sync(0xffffffffu, t.x, l0);
+        t0.y = __shfl_sync(0xffffffffu, t.y, l0);
+        t1.x = __shfl_sync(0xffffffffu, t.x, l0 + 1);
+        t1.y = __shfl_sync(0xffffffffu, t.y, l0 + 1);
+        t2.x = __shfl_sync(0xffffffffu, t.x, l0 + 2);
+        t2.y = __shfl_sync(0xffffffffu, t.y, l0 + 2);
+        const double2 det = xcadd(xcadd(t0, t1), t2);
+        dre = det.x;
+        double2 a[3], b[3];
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            a[k] = X[(3 * ca + k) * N];
+            b[k] = X[(3 * cb + k) * N];
+        }
+        __syncwarp();
+        if (det.x != 0.0 || det.y != 0.0) {
+            const SmithDen sd = smith_prepare(det);
+#pragma unroll
+            for (int k = 0; k < 3; k++)
+                v[k] = smith_div(xcsub(xcmul(a[(k + 1) % 3], b[(k + 2) % 3]), xcmul(a[(k + 2) % 3], b[(k + 1) % 3])), det,
+                                 sd);
+        } else {
+            v[0] = v[1] = v[2] = cz();
+        }
+    }
+    // a site whose determinant has no real part takes no hits, its lanes the barriers all the same
+    for (unsigned h = 1; h <= hits; h++) {
+        double2 w1[3] = {w[0], w[1], w[2]};
+        col_sub_los_alamos<0, 1>(w1, X, c);
+        col_sub_los_alamos<0, 2>(w1, X, c);
+        col_sub_los_alamos<1, 2>(w1, X, c);
+        if (dre != 0.0)
+#pragma unroll
+            for (int r = 0; r < 3; r++) w[r] = w1[r];
+    }
+#pragma unroll
+    for (int r = 0; r < 3; r++) X[(3 * r + c) * N] = w[r];
+    __syncwarp();
+    M3 m;
+    double2 t[3];
+    load_m(X, N, m);
+    col_prod(m, v, t);
+#pragma unroll
+    for (int r = 0; r < 3; r++)
+        v[r] = r == c ? make_double2(xa(1.0, xm(omega, xs(t[r].x, 1.0))), xm(omega, t[r].y))
+                      : make_double2(xm(omega, t[r].x), xm(omega, t[r].y));
+    // xproject
+    {
+        int st = col_normalize(v[0], l0);
+        __syncwarp();
+        X[c * N] = v[0];
+        X[(3 + c) * N] = v[1];
+        __syncwarp();
+        const double2 va = X[ca * N], vb = X[cb * N];
+        v[2] = col_cross(va, vb, X[(3 + ca) * N], X[(3 + cb) * N]);
+        st |= col_normalize(v[2], l0);
+        X[(6 + c) * N] = v[2];
+        __syncwarp();
+        v[1] = col_cross(X[(6 + ca) * N], X[(6 + cb) * N], va, vb);
+        if (st)
+#pragma unroll
+            for (int r = 0; r < 3; r++) v[r] = make_double2(r == c ? 1.0 : 0.0, 0.0);
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < 3; r++) X[(3 * r + c) * N] = v[r];
+        __syncwarp();
+    }
+    // m: the update, ud: its row c conjugated
+    load_m(X, N, m);
+    double2 ud[3], b[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) ud[k] = cconj(X[(3 * c + k) * N]);
+    double2 gc[3];
+#pragma unroll
+    for (int r = 0; r < 3; r++) gc[r] = g[gidx(l, par, 3 * r + c, si)];
+#pragma unroll 1
+    for (int d = 0; d < 3; d++) {
+        const uint32_t bk = d == 0 ? ib[0] : (d == 1 ? ib[1] : ib[2]);
+        const double2 *q = sm + (2 * d) * 9 * N;
+#pragma unroll
+        for (int k = 0; k < 3; k++) b[k] = q[(3 * k + c) * N];
+        col_prod(m, b, t);
+        if (keep)
+#pragma unroll
+            for (int r = 0; r < 3; r++) u[uidx(l, d, par, 3 * r + c, si)] = t[r];
+        q += 9 * N;
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+            double2 a = cz();
+#pragma unroll
+            for (int k = 0; k < 3; k++) a = xcadd(a, xcmul(q[(3 * r + k) * N], ud[k]));
+            if (keep) u[uidx(l, d, op, 3 * r + c, bk)] = a;
+        }
+    }
+    col_prod(m, gc, t);
+    if (keep)
+#pragma unroll
+        for (int r = 0; r < 3; r++) g[gidx(l, par, 3 * r + c, si)] = t[r];
+}
+
 template <int BLOCK, int MINB>
 static void launch_exact_staged(const Lat &l, double2 *u, double2 *g, int par, double omega, unsigned hits,
                                 cudaStream_t s, const unsigned *stop) {
@@ -240,6 +483,17 @@ __global__ void __launch_bounds__(LEVEL_BLOCK, 8) k_sweep_exact_pieces(double2 *
     }
 }
 
+template <bool CB>
+static void launch_exact_cols(const Lat &l, double2 *u, double2 *g, int sweep, int level, double omega, unsigned hits,
+                              cudaStream_t s, const unsigned *stop) {
+    constexpr size_t bytes = (size_t)COL_UNITS * sizeof(double2);
+    static std::atomic<unsigned long long> done{0};
+    smem_attr_once(done, k_sweep_exact_cols<CB>, bytes);
+    const uint32_t n = CB ? l.vh : odd_level_count(l, level) * (uint32_t)l.nt;
+    launch_early(k_sweep_exact_cols<CB>, (n + COL_SITES - 1) / COL_SITES, 32, bytes, s, u, g, l, sweep, level, omega, hits,
+                 stop);
+}
+
 int exact_num_shapes() { return 5; }
 
 // returns the number of kernels launched
@@ -247,6 +501,12 @@ int launch_sweep_exact(double2 *u, double2 *g, const Lat &l, int sweep, double o
                         cudaStream_t s, int shape, const unsigned *stop) {
     if (l.cb) {
         int par = sweep & 1;  // BLACKRED_SWEEP: even sites on even sweeps (gauge_fixing.c:42)
+        // three lanes to a site while a thread to a site leaves most of an SM's places for
+        // warps empty (six or fewer of its warps per SM); see k_sweep_exact_cols
+        if (l.vh <= 6u * 148u * 32u) {
+            launch_exact_cols<true>(l, u, g, sweep, 0, omega, hits, s, stop);
+            return 1;
+        }
         switch (shape) {
             case 1:
                 launch_early(k_sweep_exact<128, 3>, (l.vh + 127) / 128, 128, 0, s, u, g, l, par, omega, hits, stop);
@@ -269,6 +529,12 @@ int launch_sweep_exact(double2 *u, double2 *g, const Lat &l, int sweep, double o
         constexpr size_t bytes = (size_t)6 * 9 * LEVEL_BLOCK * sizeof(double2);
         static std::atomic<unsigned long long> done{0};
         smem_attr_once(done, k_sweep_exact_level, bytes);
+        // three lanes to a site as for even ns; it takes its levels one launch each
+        if (l.ns > 1 && l.v / 2 <= 6u * 148u * 32u) {
+            for (int level = 0; level < 4; level++)
+                launch_exact_cols<false>(l, u, g, sweep, level, omega, hits, s, stop);
+            return 4;
+        }
         // one launch up to two waves of its warps (8 per SM), where a launch is a warp's
         // chain of instructions; level by level where the sectors of whole rows count
         if (l.ns > 1 && OddPieces(l).count() * (uint32_t)l.nt <= 2 * 8 * 148) {

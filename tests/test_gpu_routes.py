@@ -1,0 +1,71 @@
+"""Half-sweeps on every route that the launch rules choose between, by lattice size: each
+against the CPU oracle's half-sweeps of the same links."""
+import numpy as np
+import pytest
+
+import gfc
+import oracle_ref as orc
+
+pytestmark = pytest.mark.gpu
+
+
+def swept(ns, nt, prec, n, seed=71, scale=0.6, hits=2):
+    """(links, G) after n half-sweeps on the GPU and by the oracle."""
+    U = gfc.synth_config(ns, nt, seed, scale)
+    orc.reunitarize(U)
+    with gfc.Lattice(ns, nt) as lat:
+        lat.upload_links(U, 8, False)
+        lat.set_identity_gt()
+        lat.halfsweeps(0, n, omega=1.95, hits=hits, precision=prec)
+        got = lat.download_links(), lat.download_gt()
+        assert lat.status() == 0
+    V = ns ** 3 * nt
+    G = np.zeros(V * 18)
+    G.reshape(V, 9, 2)[:, [0, 4, 8], 0] = 1.0
+    for k in range(n):
+        orc.halfsweep(U, G, ns, nt, k, float(np.float32(1.95)), hits)
+    U4, got4 = U.reshape(V, 4, 18), got[0].reshape(V, 4, 18)
+    return U4[:, 1:], G, got4[:, 1:], got[1]
+
+
+# three lanes to a site (sites not a multiple of a warp's ten; odd ns by level), one launch
+# over the components of odd ns, one launch per level, a thread to a site
+@pytest.mark.parametrize("ns,nt,hits", [(2, 3, 2), (4, 1, 3), (6, 5, 1), (14, 20, 2), (14, 22, 2),
+                                        (3, 4, 2), (5, 3, 3), (13, 5, 2), (15, 18, 2), (21, 20, 2)])
+def test_exact_half_sweeps_bit_for_bit(ns, nt, hits):
+    U, G, Ug, Gg = swept(ns, nt, gfc.PREC_FP64_EXACT, 3, hits=hits)
+    assert np.array_equal(Gg, G)
+    assert np.array_equal(Ug, U)
+
+
+# each update multiplies a link by a unit matrix computed to rounding: three half-sweeps of
+# O(100) operations on entries below one stay within 1e-13
+@pytest.mark.parametrize("ns,nt,hits", [(2, 3, 2), (4, 1, 3), (6, 5, 1), (12, 14, 2), (14, 22, 2),
+                                        (3, 4, 2), (5, 3, 3), (9, 8, 2), (13, 5, 2), (15, 18, 2)])
+def test_fast_half_sweeps(ns, nt, hits):
+    U, G, Ug, Gg = swept(ns, nt, gfc.PREC_FP64_FAST, 3, hits=hits)
+    assert np.abs(Gg - G).max() < 1e-13
+    assert np.abs(Ug - U).max() < 1e-13
+
+
+@pytest.mark.parametrize("ns,nt", [(6, 4), (9, 7), (12, 5)])
+def test_copies_from_and_to_ordinary_memory(ns, nt):
+    """Pieces of 1 MB: below one, several and a remainder, against page-locked memory."""
+    rng = np.random.default_rng(ns)
+    U, G = rng.standard_normal(ns ** 3 * nt * 72), rng.standard_normal(ns ** 3 * nt * 18)
+    pin = gfc.PinnedBuffer(U.nbytes)
+    with gfc.Lattice(ns, nt) as lat:
+        lat.upload_links(U)
+        lat.upload_gt(G)
+        assert np.array_equal(lat.download_links(out=pin.view(np.float64)), U)
+        assert np.array_equal(lat.download_links(), U)
+        assert np.array_equal(lat.download_gt(), G)
+        assert np.array_equal(lat.download_gt(4), G.astype(np.float32))
+    with gfc.Batch(ns ** 3 * nt, max_slots=1, max_nt=nt) as b:
+        s = b.add(ns, nt)
+        links = gfc.synth_config(ns, nt, 5, 0.5)
+        b.upload(s, links)
+        a = b.download_links(s)
+        pin.view(np.float64)[:] = links
+        b.upload(s, pin.view(np.float64))
+        assert np.array_equal(a, b.download_links(s))
