@@ -62,6 +62,11 @@ static void ctx_free(gfc_ctx *c) {
     cudaFree(c->e2_hist);
     cudaFree(c->tickets);
     cudaFree(c->ring);
+    cudaFreeHost(c->hlook);
+    if (c->ev_chunk) cudaEventDestroy(c->ev_chunk);
+    for (int k = 0; k < 2; k++)
+        if (c->ev_look[k]) cudaEventDestroy(c->ev_look[k]);
+    if (c->sl) cudaStreamDestroy(c->sl);
     for (int k = 0; k < 2; k++) {
         cudaFree(c->dstage[k]);
         if (c->ev_copy[k]) cudaEventDestroy(c->ev_copy[k]);

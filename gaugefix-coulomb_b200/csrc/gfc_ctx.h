@@ -55,6 +55,10 @@ struct gfc_ctx {
     int blk32_slices = 0, blk32_sweeps = 1;
     double *ring = nullptr;       // per-slice e2 partials of the last half-sweeps
     int ring_n = 0;
+    // a fix's stop word and e2 read back beside the sweeps that follow (run_until)
+    cudaStream_t sl = nullptr;
+    cudaEvent_t ev_chunk = nullptr, ev_look[2] = {nullptr, nullptr};
+    double *hlook = nullptr;      // pinned, [2][4]: e2 pair, stop word
 };
 
 namespace gfc {
