@@ -48,6 +48,29 @@ def test_fast_half_sweeps(ns, nt, hits):
     assert np.abs(Ug - U).max() < 1e-13
 
 
+# a lattice of 80 to 300 MB of working fields sweeps with L2 hints (the fully staged
+# launch shapes) or without (shape 15): nine half-sweeps with a reunitarisation after every
+# fourth, folded into the sweep or not; FP32 rounds at 6e-8 per operation, some hundred
+# operations per entry
+@pytest.mark.parametrize("ns,nt,prec,tol", [(20, 28, gfc.PREC_FP64_FAST, 1e-13), (24, 33, gfc.PREC_MIXED, 3e-5)])
+def test_l2_hints_change_nothing(ns, nt, prec, tol):
+    U = gfc.synth_config(ns, nt, 72, 0.6)
+    p = gfc.default_params(tolerance=1e-30, max_sweeps_to_fix=9, sweeps_to_reunitarization=4)
+    o = gfc.options(precision=prec, stop_rule=gfc.STOP_EVERY, switch_e2=1e-29,
+                    fp32_refresh=4 if prec == gfc.PREC_MIXED else 0)
+    G = []
+    with gfc.Lattice(ns, nt, mixed=prec == gfc.PREC_MIXED) as lat:
+        for shape in (10, 15):
+            lat.set_shapes(fast64=shape, fast32=shape)
+            lat.upload_links_reunit(U)
+            rc, _ = lat.fix(p, o)
+            assert rc == gfc.FIX_NOT_CONVERGED and lat.status() == 0
+            G.append(lat.download_gt())
+    assert np.abs(G[0] - G[1]).max() <= tol
+    # the half-sweeps have done something
+    assert np.abs(G[0].reshape(-1, 9, 2)[:, 0, 0] - 1).max() > 0.1
+
+
 @pytest.mark.parametrize("ns,nt", [(6, 4), (9, 7), (12, 5)])
 def test_copies_from_and_to_ordinary_memory(ns, nt):
     """Pieces of 1 MB: below one, several and a remainder, against page-locked memory."""
