@@ -123,7 +123,12 @@ __device__ __forceinline__ void diva_add(DivA &d, const M3 &f, const M3 &r) {
 __device__ __forceinline__ void diva_densities(const DivA &d, double &e2, double &th) {
     const double c2 = xs(d.h[0], d.h[1]);
     const double c7 = xd(xs(xa(d.h[0], d.h[1]), xm(2.0, d.h[2])), __dsqrt_rn(3.0));
-    double s = xm(d.p[0], d.p[0]);
+    // NaN where an entry off the diagonal is not finite (the reference multiplies it by
+    // (-0, -1/2), and 0 times infinity is NaN), 0 elsewhere
+    double z = 0.0;
+#pragma unroll
+    for (int k = 0; k < 3; k++) z = __fma_rn(0.0, d.q[k], __fma_rn(0.0, d.p[k], z));
+    double s = xa(z, xm(d.p[0], d.p[0]));
     s = xa(s, xm(d.q[0], d.q[0]));
     s = xa(s, xm(c2, c2));
     s = xa(s, xm(d.p[1], d.p[1]));
@@ -137,7 +142,7 @@ __device__ __forceinline__ void diva_densities(const DivA &d, double &e2, double
         n[k] = xm(0.25, xa(xm(d.p[k], d.p[k]), xm(d.q[k], d.q[k])));
         m[k] = xm(d.h[k], d.h[k]);
     }
-    th = xa(xa(xa(xa(m[0], n[0]), n[1]), xa(xa(n[0], m[1]), n[2])), xa(xa(n[1], n[2]), m[2]));
+    th = xa(xa(xa(xa(xa(z, m[0]), n[0]), n[1]), xa(xa(n[0], m[1]), n[2])), xa(xa(n[1], n[2]), m[2]));
 }
 
 }  // namespace gfc

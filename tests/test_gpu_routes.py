@@ -92,3 +92,28 @@ def test_copies_from_and_to_ordinary_memory(ns, nt):
         pin.view(np.float64)[:] = links
         b.upload(s, pin.view(np.float64))
         assert np.array_equal(a, b.download_links(s))
+
+
+# an entry that is not finite, on or off the diagonal: a number or NaN where the reference's
+# operations give one or the other; number for number the rounding of sums of 54 or 128
+# sites of a hundred operations each
+@pytest.mark.parametrize("ns", [3, 4])
+@pytest.mark.parametrize("a,b,part", [(0, 1, 0), (2, 0, 1), (1, 1, 1), (0, 0, 0), (2, 2, 1)])
+@pytest.mark.parametrize("x", [0.25, np.inf, -np.inf, np.nan])
+def test_observables_of_links_that_are_not_finite(ns, a, b, part, x):
+    import ctypes
+
+    import torch
+    nt = 2
+    U = gfc.synth_config(ns, nt, 73, 0.6)
+    U.reshape(nt, ns, ns, ns, 4, 3, 3, 2)[1, 0, 1, 2, 2, a, b, part] = x
+    want = orc.e2(U, ns, nt), orc.theta(U, ns, nt)
+    assert np.isnan(want).all() == (not np.isfinite(x) and (a, b, part) != (0, 0, 0))
+    with gfc.Lattice(ns, nt) as lat:
+        lat.upload_links(U, 8, False)
+        np.testing.assert_allclose(lat.e2_theta(), want, rtol=1e-12)
+    d = torch.from_numpy(U).cuda()
+    torch.cuda.synchronize()
+    e2, th = ctypes.c_double(), ctypes.c_double()
+    assert gfc.lib.gfc_e2_theta_device_noalloc(ns, nt, d.data_ptr(), None, ctypes.byref(e2), ctypes.byref(th)) == gfc.GFC_OK
+    np.testing.assert_allclose((e2.value, th.value), want, rtol=1e-12)
