@@ -32,6 +32,8 @@
 #include "gfc.h"
 #include "gfc_ctx.h"
 #include "gfc_device.cuh"
+#include "gfc_internal.h"
+#include "gfc_reduce.cuh"
 
 namespace gfc {
 
@@ -39,33 +41,11 @@ static __device__ __align__(256) double g_noalloc_scratch[GFC_NOALLOC_SCRATCH_DO
 
 namespace {
 
-constexpr int NA_BLOCK = 256;
+constexpr int NA_BLOCK = 64, NA_MIN_BLOCKS = 8;   // k_obs_partials_noalloc
+constexpr int NA_FIN_BLOCK = 256;                  // k_finalize_noalloc
 constexpr int NA_MAX_DEVICES = 64;
 std::mutex na_mutex;
 double *na_scratch[NA_MAX_DEVICES] = {nullptr};
-
-// A_mu = -(i/2) traceless(U - U^dagger), rounded like the reference
-// (subtractionHermConjTrless3x3 SU3_ops.c:322-372, calculateA four_potential.c:35-66)
-__device__ __forceinline__ void na_calc_A(const M3 &u, M3 &A) {
-    M3 d;
-    double2 tr = cz();
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        d.e[EL(a, a)] = make_double2(0.0, xm(2.0, u.e[EL(a, a)].y));
-        tr = xcadd(tr, d.e[EL(a, a)]);
-    }
-    tr = make_double2(xd(tr.x, 3.0), xd(tr.y, 3.0));
-#pragma unroll
-    for (int a = 0; a < 3; a++) d.e[EL(a, a)] = xcsub(d.e[EL(a, a)], tr);
-#pragma unroll
-    for (int a = 0; a < 3; a++)
-#pragma unroll
-        for (int b = 0; b < 3; b++)
-            if (a != b) d.e[EL(a, b)] = xcsub(u.e[EL(a, b)], cconj(u.e[EL(b, a)]));
-    const double2 al = make_double2(-0.0, -0.5);
-#pragma unroll
-    for (int k = 0; k < 9; k++) A.e[k] = xcmul(al, d.e[k]);
-}
 
 __device__ __forceinline__ void na_load_aos(const double2 *__restrict__ u, uint32_t L, int mu, M3 &m) {
     const double2 *p = u + ((size_t)L * 4 + mu) * 9;
@@ -78,48 +58,31 @@ __device__ __forceinline__ void na_load_aos(const double2 *__restrict__ u, uint3
 __device__ __forceinline__ void na_site(const double2 *__restrict__ u, const Lat &l, uint32_t L, double &e2,
                                         double &th) {
     Coord c = coord_lex(l, L);
-    M3 dA;
-#pragma unroll
-    for (int k = 0; k < 9; k++) dA.e[k] = cz();
+    DivA dA;
+    diva_zero(dA);
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-        M3 f, r, A1, A2;
+        M3 f, r;
         na_load_aos(u, L, d + 1, f);
         na_load_aos(u, back_L(l, c, d), d + 1, r);
-        na_calc_A(f, A1);
-        na_calc_A(r, A2);
-#pragma unroll
-        for (int k = 0; k < 9; k++) dA.e[k] = xcadd(dA.e[k], xcsub(A1.e[k], A2.e[k]));
+        diva_add(dA, f, r);
     }
-    const double2 *m = dA.e;
-    double cc[8];
-    cc[0] = xa(m[EL(0, 1)].x, m[EL(1, 0)].x);
-    cc[1] = xa(-m[EL(0, 1)].y, m[EL(1, 0)].y);
-    cc[2] = xs(m[EL(0, 0)].x, m[EL(1, 1)].x);
-    cc[3] = xa(m[EL(0, 2)].x, m[EL(2, 0)].x);
-    cc[4] = xa(-m[EL(0, 2)].y, m[EL(2, 0)].y);
-    cc[5] = xa(m[EL(1, 2)].x, m[EL(2, 1)].x);
-    cc[6] = xa(-m[EL(1, 2)].y, m[EL(2, 1)].y);
-    cc[7] = xd(xs(xa(m[EL(0, 0)].x, m[EL(1, 1)].x), xm(2.0, m[EL(2, 2)].x)), __dsqrt_rn(3.0));
-    double s = 0.0;
-#pragma unroll
-    for (int a = 0; a < 8; a++) s = xa(s, xm(cc[a], cc[a]));
-    e2 = s;
-    double t = 0.0;
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        double2 sa = cz();
-#pragma unroll
-        for (int k = 0; k < 3; k++) sa = xcadd(sa, xcmul(m[EL(a, k)], cconj(m[EL(a, k)])));
-        t = xa(t, sa.x);
-    }
-    th = t;
+    diva_densities(dA, e2, th);
 }
 
-// grid (nbx, nt): block bx of timeslice t writes scratch[(t*nbx + bx)*2 + {0,1}]
-__global__ void __launch_bounds__(NA_BLOCK) k_obs_partials_noalloc(const double2 *__restrict__ u, Lat l,
-                                                                   double *__restrict__ scratch) {
+// grid (nbx, nt): block bx of timeslice t writes scratch[(t*nbx + bx)*2 + {0,1}].  Bound by
+// the latency and the tags of its loads: lanes lie 576 bytes apart, so each of a site's 54
+// loads touches 32 lines.  So what counts is warps in flight: with DivA's 9 sums instead
+// of whole matrices 128 registers do (16 warps per SM), and blocks of two warps, up to two
+// rounds of them, leave the shortest last wave.  A call, copy and synchronisation
+// included, at 8^3 x 16 / 16^3 x 32 / 24^3 x 48 / 32^3 x 64: 20.1 / 45.4 / 132 / 336 us;
+// 128-thread blocks 22.8 / 44.4 / 132 / 361, at 166 registers 21.9 / 47.1 / 133 / 370;
+// 256-thread blocks on whole matrices 30.7 / 56.0 / 147 / 377.
+__global__ void __launch_bounds__(NA_BLOCK, NA_MIN_BLOCKS) k_obs_partials_noalloc(const double2 *__restrict__ u,
+                                                                                  Lat l,
+                                                                                  double *__restrict__ scratch) {
     __shared__ double sh[2][NA_BLOCK / 32];
+    grid_wait();
     const uint32_t t = blockIdx.y;
     double v0 = 0.0, v1 = 0.0;
     for (uint32_t k = blockIdx.x * NA_BLOCK + threadIdx.x; k < l.vs; k += gridDim.x * NA_BLOCK) {
@@ -151,19 +114,20 @@ __global__ void __launch_bounds__(NA_BLOCK) k_obs_partials_noalloc(const double2
     }
 }
 
-// one block: sums the nparts partial pairs in index order into scratch[res_off + {0,1}]
-__global__ void __launch_bounds__(NA_BLOCK) k_finalize_noalloc(double *__restrict__ scratch, uint32_t nparts,
-                                                               uint32_t res_off) {
-    __shared__ double acc[2][NA_BLOCK];
+// one block (launch_early): sums the nparts partial pairs in index order into scratch[res_off + {0,1}]
+__global__ void __launch_bounds__(NA_FIN_BLOCK) k_finalize_noalloc(double *__restrict__ scratch, uint32_t nparts,
+                                                                   uint32_t res_off) {
+    grid_wait();
+    __shared__ double acc[2][NA_FIN_BLOCK];
     double s0 = 0.0, s1 = 0.0;
-    for (uint32_t p = threadIdx.x; p < nparts; p += NA_BLOCK) {
+    for (uint32_t p = threadIdx.x; p < nparts; p += NA_FIN_BLOCK) {
         s0 += scratch[2 * (size_t)p];
         s1 += scratch[2 * (size_t)p + 1];
     }
     acc[0][threadIdx.x] = s0;
     acc[1][threadIdx.x] = s1;
     __syncthreads();
-    for (int w = NA_BLOCK / 2; w > 0; w >>= 1) {
+    for (int w = NA_FIN_BLOCK / 2; w > 0; w >>= 1) {
         if ((int)threadIdx.x < w) {
             acc[0][threadIdx.x] += acc[0][threadIdx.x + w];
             acc[1][threadIdx.x] += acc[1][threadIdx.x + w];
@@ -236,7 +200,7 @@ extern "C" int gfc_e2_theta_device_noalloc(int ns, int nt, const double *u_dev, 
     }
     const Lat l = make_lat(ns, nt);
     uint32_t nbx = (l.vs + NA_BLOCK - 1) / NA_BLOCK;
-    const uint32_t want = (4u * 148u + (uint32_t)nt - 1) / (uint32_t)nt;
+    const uint32_t want = (2u * NA_MIN_BLOCKS * 148u + (uint32_t)nt - 1) / (uint32_t)nt;
     if (nbx > want) nbx = want;
     if (nbx < 1) nbx = 1;
     const uint64_t nparts = (uint64_t)nbx * (uint64_t)nt;
@@ -252,7 +216,7 @@ extern "C" int gfc_e2_theta_device_noalloc(int ns, int nt, const double *u_dev, 
     if (rc) return rc;
     cudaStream_t s = (cudaStream_t)stream;
     k_obs_partials_noalloc<<<dim3(nbx, nt), NA_BLOCK, 0, s>>>((const double2 *)u_dev, l, scratch);
-    k_finalize_noalloc<<<1, NA_BLOCK, 0, s>>>(scratch, (uint32_t)nparts, (uint32_t)res_off);
+    launch_early(k_finalize_noalloc, 1, NA_FIN_BLOCK, 0, s, scratch, (uint32_t)nparts, (uint32_t)res_off);
     GFC_CHECK(cudaGetLastError());
     double h[2];
     GFC_CHECK(cudaMemcpyAsync(h, scratch + res_off, sizeof h, cudaMemcpyDeviceToHost, s));

@@ -117,3 +117,22 @@ def test_observables_of_links_that_are_not_finite(ns, a, b, part, x):
     e2, th = ctypes.c_double(), ctypes.c_double()
     assert gfc.lib.gfc_e2_theta_device_noalloc(ns, nt, d.data_ptr(), None, ctypes.byref(e2), ctypes.byref(th)) == gfc.GFC_OK
     np.testing.assert_allclose((e2.value, th.value), want, rtol=1e-12)
+
+
+# blocks of 64 sites of a timeslice: one site, a part of a block, whole blocks, more than
+# 2368 blocks (a loop inside them), more than 2368 timeslices (a block to each); sums of at
+# most 1.8e5 sites in two orders
+@pytest.mark.parametrize("ns,nt", [(1, 1), (3, 2), (4, 3), (5, 1), (54, 1), (2, 2400)])
+def test_e2_of_caller_owned_links_against_the_context(ns, nt):
+    import ctypes
+
+    import torch
+    U = np.random.default_rng(ns).standard_normal(ns ** 3 * nt * 72)
+    with gfc.Lattice(ns, nt) as lat:
+        lat.upload_links(U, 8, False)
+        want = lat.e2_theta()
+    d = torch.from_numpy(U).cuda()
+    torch.cuda.synchronize()
+    e2, th = ctypes.c_double(), ctypes.c_double()
+    assert gfc.lib.gfc_e2_theta_device_noalloc(ns, nt, d.data_ptr(), None, ctypes.byref(e2), ctypes.byref(th)) == gfc.GFC_OK
+    np.testing.assert_allclose((e2.value, th.value), want, rtol=1e-12)
